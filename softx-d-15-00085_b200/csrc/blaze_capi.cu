@@ -8,6 +8,7 @@
 // and a step is a fixed sequence of kernel launches on one stream.
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <cstddef>
 #include <cstdio>
 #include <cstring>
@@ -17,7 +18,6 @@
 #include "blaze_dem.h"
 #include "dem_kernels.cuh"
 #include "poly_kernels.cuh"
-#include "radix_sort.cuh"
 
 using namespace blaze;
 
@@ -62,9 +62,7 @@ struct blaze_sim {
   StateBuf S[3]{};  // S[0], S[1] ping-pong, S[2] sorted gather target
   OrderBuf ob{};
   int cur = 0;      // S[cur] holds the current state
-  RadixSortBuffers rs{};
-  uint32_t* cstart = nullptr;
-  uint32_t* cend = nullptr;
+  CellSort cs{};
   NbrList nl{};
   StepCtl* ctl = nullptr;
   StepCtl* h_ctl = nullptr;  // pinned mirror
@@ -83,8 +81,7 @@ struct blaze_sim {
   int* d_rb = nullptr;                 // per graph step: nonzero when that step re-sorted
   uint32_t* d_chk = nullptr;           // list-check maxima slots (StepCtl::chk)
   bool spin_free = false;              // rotation off and every angular velocity zero
-  int key_bits = 1;
-  uint32_t cells_cap = 0;   // entries allocated in cstart / cend
+  uint32_t tiles_cap = 0;   // tiles of cells allocated in cs
   long long steps = 0;
   // with a skin, steps below this index each end with a list check (from a
   // forced re-sort to the next multiple of kListCheckEvery; see force_check)
@@ -218,6 +215,17 @@ void build_params(blaze_sim* s) {
   }
   P.max_nbr = s->opt.max_nbr;
   P.skin = s->opt.skin;
+  // The neighbour search may skip cells out of a particle's reach only where
+  // that cannot drop a pair the full search finds: a partner must lie within
+  // one cell, and no cell scanned may share its hash value (x + z ncz +
+  // y ncx ncz) with another one within reach, which would list the partner
+  // through that cell too.  Six cells along x and z put such cells at least
+  // four apart.
+  float rmax = 0.0f;
+  for (int t = 0; t < s->n_p; ++t) rmax = std::max(rmax, s->p[t].radius);
+  const float edge = std::min(P.cell.x, std::min(P.cell.y, P.cell.z));
+  const bool near_only = nx >= 6 && nz >= 6 && edge >= 2.0f * rmax + P.skin;
+  P.r_max = near_only ? rmax : std::numeric_limits<float>::infinity();
 }
 
 // World objects -> the wall program, in world-object order
@@ -453,24 +461,25 @@ int upload_params(blaze_sim* s) {
   return upload_walls(s);
 }
 
-// The cell table and the sort's key width for the current grid (the list
-// grid with a skin, the project's without); reallocated when the grid grows.
+// The cell table of the current grid (the list grid with a skin, the
+// project's without); reallocated when the grid grows.
 int alloc_cells(blaze_sim* s) {
-  const uint32_t nt = s->hp.ncell_tab;
-  const uint32_t top = nt + 1u;
-  s->key_bits = 1;
-  while (s->key_bits < 32 && (top >> s->key_bits) != 0) s->key_bits++;
-  if (nt > s->cells_cap) {
-    if (s->cstart) CK(cudaFree(s->cstart));
-    if (s->cend) CK(cudaFree(s->cend));
-    s->cstart = s->cend = nullptr;
-    s->cells_cap = 0;
-    CK(dalloc(&s->cstart, nt));
-    CK(dalloc(&s->cend, nt));
-    s->cells_cap = nt;
+  const uint32_t tiles = cell_tiles(s->hp.ncell_tab);
+  s->cs.ncell = s->hp.ncell_tab;
+  if (tiles > s->tiles_cap) {
+    for (uint32_t** q : {&s->cs.cnt, &s->cs.start, &s->cs.tile}) {
+      if (*q) CK(cudaFree(*q));
+      *q = nullptr;
+    }
+    s->tiles_cap = 0;
+    CK(dalloc(&s->cs.cnt, (size_t)tiles * kTileCells));
+    CK(dalloc(&s->cs.start, (size_t)tiles * kTileCells));
+    CK(dalloc(&s->cs.tile, (size_t)tiles + 1));
+    s->tiles_cap = tiles;
   }
-  CK(cudaMemset(s->cstart, 0xff, sizeof(uint32_t) * nt));
-  CK(cudaMemset(s->cend, 0xff, sizeof(uint32_t) * nt));
+  CK(cudaMemset(s->cs.cnt, 0, sizeof(uint32_t) * (size_t)tiles * kTileCells));
+  CK(cudaMemset(s->cs.start, 0, sizeof(uint32_t) * (size_t)tiles * kTileCells));
+  CK(cudaMemset(s->cs.tile, 0, sizeof(uint32_t) * ((size_t)tiles + 1)));
   return 0;
 }
 
@@ -537,16 +546,17 @@ int alloc_capture(blaze_sim* s) {
 }
 
 // --------------------------------------------------------------- the step
+// kernels of one re-sort: key and count, scan, place, move, neighbour list
+constexpr int kRebuildKernels = 3 + kCellSortKernels;
+
 int enqueue_rebuild(blaze_sim* s, const int* gate, cudaStream_t st) {
   const int n = s->n_max;
-  launch_hash(s->dp, s->S[s->cur], s->ob, n, s->rs.keys[0], s->ctl, gate, st);
-  const int res = radix_sort_pairs(s->rs, n, s->key_bits, true, gate, st);
-  const size_t cbytes = sizeof(uint32_t) * s->hp.ncell_tab;
-  CK(cudaMemsetAsync(s->cstart, 0xff, cbytes, st));
-  launch_reorder(s->S[s->cur], s->S[2], s->ob, n, s->rs.keys[res], s->rs.vals[res], s->cstart,
-                 s->cend, s->hp.ncell_tab, s->n_d > 0, s->nl.flat_n, s->ctl, gate, st);
-  launch_nlist(s->dp, s->S[2], n, s->cstart, s->cend, s->nl, s->ctl, gate, st);
-  s->last_launches += 3 + 3 * std::max(1, (s->key_bits + kRadixBits - 1) / kRadixBits);
+  launch_hash(s->dp, s->S[s->cur], s->ob, n, s->cs, s->ctl, gate, st);
+  cell_scan_place(s->cs, n, nullptr, gate, st);
+  launch_reorder(s->S[s->cur], s->S[2], s->ob, n, s->cs, s->n_d > 0, s->nl.flat_n, s->ctl, gate,
+                 st);
+  launch_nlist(s->dp, s->S[2], n, s->cs.start, s->nl, s->ctl, gate, st);
+  s->last_launches += kRebuildKernels;
   return 0;
 }
 
@@ -1039,8 +1049,9 @@ void free_sim(blaze_sim* s) {
   if (!s) return;
   auto f = [](void* p) { if (p) cudaFree(p); };
   for (int b = 0; b < 3; ++b) { f(s->S[b].pos); f(s->S[b].vel); f(s->S[b].angv); }
-  for (int b = 0; b < 2; ++b) { f(s->ob.pid[b]); f(s->ob.lift[b]); f(s->rs.keys[b]); f(s->rs.vals[b]); }
-  f(s->rs.counts); f(s->rs.totals); f(s->cstart); f(s->cend); f(s->nl.idx); f(s->nl.cnt);
+  for (int b = 0; b < 2; ++b) { f(s->ob.pid[b]); f(s->ob.lift[b]); }
+  f(s->cs.key); f(s->cs.slot); f(s->cs.member); f(s->cs.cnt); f(s->cs.start); f(s->cs.tile);
+  f(s->cs.spec); f(s->nl.idx); f(s->nl.cnt);
   f(s->ctl); f(s->d_rb); f(s->d_chk); f(s->dp); f(s->d_ops); f(s->d_wall_off); f(s->d_wall_idx);
   f(s->d_tally); f(s->d_eb); f(s->d_epart);
   f(s->cap.f_pp); f(s->cap.t_pp); f(s->cap.f_w); f(s->cap.t_w); f(s->cap.f_l); f(s->cap.t_l);
@@ -1198,14 +1209,11 @@ int create_impl(blaze_sim** out, const WOBJ* w, int n_w, const POBJ* p, int n_p,
   for (int b = 0; b < 2; ++b) {
     CKF(dalloc(&s->ob.pid[b], n));
     CKF(dalloc(&s->ob.lift[b], n));
-    CKF(dalloc(&s->rs.keys[b], n));
-    CKF(dalloc(&s->rs.vals[b], n));
   }
-  const int tiles = (n + kTileKeys - 1) / kTileKeys;
-  s->rs.max_n = n;
-  s->rs.max_tiles = tiles;
-  CKF(dalloc(&s->rs.counts, (size_t)kRadixDigits * std::max(tiles, 1)));
-  CKF(dalloc(&s->rs.totals, kRadixDigits));
+  CKF(dalloc(&s->cs.key, n));
+  CKF(dalloc(&s->cs.slot, n));
+  CKF(dalloc(&s->cs.member, n));
+  CKF(dalloc(&s->cs.spec, (size_t)2 * sort_blocks(n)));
   CKF(dalloc(&s->dp, 1));
   CKF(dalloc(&s->ctl, 1));
   CKF(dalloc(&s->d_rb, kGraphSteps));
@@ -1598,7 +1606,7 @@ int blaze_last_launches(blaze_sim* s) { return s ? s->last_launches : -1; }
 
 int blaze_rebuild_kernels(blaze_sim* s) {
   if (!s) return -1;
-  return 3 + 3 * std::max(1, (s->key_bits + kRadixBits - 1) / kRadixBits);
+  return kRebuildKernels;
 }
 
 int blaze_open_hatch(blaze_sim* s) {

@@ -110,6 +110,10 @@ struct SimParams {
   // neighbour list
   int max_nbr;
   float skin;
+  // the largest radius where no two cells near each other share a hash value
+  // and a contact spans at most one cell (build_params), else infinite: the
+  // neighbour search then leaves no cell out
+  float r_max;
 };
 
 // ----------------------------------------------------------------- float3 ops
@@ -126,6 +130,17 @@ __device__ __forceinline__ float3 cross3(float3 a, float3 b) {
   return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
 __device__ __forceinline__ float3 xyz(float4 a) { return f3(a.x, a.y, a.z); }
+
+// Distances from coordinate p in cell g (of nc cells of the given edge from
+// origin o) to the lower and the upper neighbour cell, less a margin for the
+// rounding of (p - o) / cell: any particle counted in that neighbour is at
+// least this far away along the axis.  The quotient is off by at most 2^-22
+// of nc cells; 0 for a coordinate that is not finite.
+__device__ __forceinline__ float2 cell_gap(float p, float o, float cell, int g, int nc) {
+  const float f = (p - o) / cell - (float)g;
+  const float m = cell * (1e-5f + 1e-6f * (float)nc);
+  return make_float2(fmaxf(f * cell - m, 0.0f), fmaxf((1.0f - f) * cell - m, 0.0f));
+}
 
 // a / b for the three components of a by one positive, normal b, correctly
 // rounded (the same numbers as three IEEE divisions), from one correctly

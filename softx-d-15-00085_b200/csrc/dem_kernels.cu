@@ -6,8 +6,9 @@
 //
 //   k_gate     one thread: latch the rebuild request for this step
 //   k_hash     cell key per particle          (BroadPhase.cuh:20-100)
-//   [radix sort, radix_sort.cu]               (BroadPhase.cuh:110-117)
-//   k_reorder  gather state into sorted order + cell start/end table
+//   [counting sort by cell and cell table, cell_sort.cu]
+//                                             (BroadPhase.cuh:110-117)
+//   k_reorder  move the state into sorted order
 //                                             (BroadPhase.cuh:126-325)
 //   k_nlist    27-cell neighbour search       (BroadPhase.cuh:335-513)
 //   k_step     particle-particle law + volume objects + world objects +
@@ -142,51 +143,54 @@ __global__ void k_gate_graph(StepCtl* ctl, cudaGraphConditionalHandle h0, int* r
 // reference's parking position max_size makes them; a live particle outside
 // the grid takes the key just below (the reference's table would be indexed
 // out of range) and raises kStatusOutOfGrid.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSortThreads)
 k_hash(const SimParams* __restrict__ P, const float4* __restrict__ pos, OrderBuf ob, int n_max,
-       uint32_t* __restrict__ keys, StepCtl* ctl, const int* gate) {
+       CellSort cs, StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_max) return;
-  const int* pid = (ctl->epoch & 1) ? ob.pid[1] : ob.pid[0];
-  uint32_t key;
+  const int i = blockIdx.x * kSortThreads + threadIdx.x;
+  const bool valid = i < n_max;
+  uint32_t key = 0;
   uint32_t st = 0;
-  // removed particles and those a fill has not reached yet stay at the end
-  if (pid[i] < 0 || i >= ctl->n_cur) {
-    key = P->ncell_tab + 1u;
-  } else {
-    const float4 p = pos[i];
-    const int3 g = grid_pos(*P, xyz(p));
-    if (in_grid(*P, g)) {
-      key = grid_hash(*P, g);
+  if (valid) {
+    const int* pid = (ctl->epoch & 1) ? ob.pid[1] : ob.pid[0];
+    // removed particles and those a fill has not reached yet stay at the end
+    if (pid[i] < 0 || i >= ctl->n_cur) {
+      key = P->ncell_tab + 1u;
     } else {
-      key = P->ncell_tab;
-      st = kStatusOutOfGrid;
+      const float4 p = pos[i];
+      const int3 g = grid_pos(*P, xyz(p));
+      if (in_grid(*P, g)) {
+        key = grid_hash(*P, g);
+      } else {
+        key = P->ncell_tab;
+        st = kStatusOutOfGrid;
+      }
     }
   }
-  keys[i] = key;
+  cell_count(cs, i, valid, key);
   flag_status(ctl, st);
 }
 
 // ------------------------------------------------------------------ reorder
-// Kernel_SortArrays + Kernel_SpatialDecomp_ReorderPDA + Kernel_SpatialDecomp_BinData
-// (BroadPhase.cuh:126-325), as one gather into the spare buffer.
-__global__ void __launch_bounds__(kThreads)
-k_reorder(StateBuf src, StateBuf dst, OrderBuf ob, int n_max,
-          const uint32_t* __restrict__ keys, const int32_t* __restrict__ perm,
-          uint32_t* __restrict__ cstart, uint32_t* __restrict__ cend, uint32_t ncell_tab,
-          int has_lift, int* flat_n, StepCtl* ctl, const int* gate) {
+// Kernel_SortArrays + Kernel_SpatialDecomp_ReorderPDA
+// (BroadPhase.cuh:126-325): every particle to its sorted position in the
+// spare buffer.  Particles are nearly in order already, so reads and writes
+// stay close to coalesced.
+__global__ void __launch_bounds__(kSortThreads)
+k_reorder(StateBuf src, StateBuf dst, OrderBuf ob, int n_max, CellSort cs, int has_lift,
+          int* flat_n, StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x * kSortThreads + threadIdx.x;
+  const bool valid = j < n_max;
   const int e = ctl->epoch & 1;
-  if (i == 0) {
+  if (j == 0) {
     // the particles removed since the last re-sort are now at the end
     ctl->n_cur -= ctl->pending_dead;
     ctl->pending_dead = 0;
     if (flat_n) *flat_n = 0;  // the contact-list kernel lists the slots anew
   }
-  if (i >= n_max) return;
-  const int j = perm[i];
+  const int i = cell_dest(cs, j, valid);
+  if (!valid) return;
   dst.pos[i] = src.pos[j];
   dst.vel[i] = src.vel[j];
   float4 w = src.angv[j];
@@ -205,11 +209,6 @@ k_reorder(StateBuf src, StateBuf dst, OrderBuf ob, int n_max,
     float4* q_dst = e ? ob.ornt[0] : ob.ornt[1];
     q_dst[i] = q_src[j];
   }
-  const uint32_t k = keys[i];
-  if (k < ncell_tab) {
-    if (i == 0 || keys[i - 1] != k) cstart[k] = (uint32_t)i;
-    if (i == n_max - 1 || keys[i + 1] != k) cend[k] = (uint32_t)i + 1u;
-  }
 }
 
 // -------------------------------------------------------------------- nlist
@@ -220,11 +219,22 @@ k_reorder(StateBuf src, StateBuf dst, OrderBuf ob, int n_max,
 // contacts-only list, bit for bit), or with a skin every pair with
 // |xi - xj| < ri + rj + skin (up to a relative 2^-20 more).  Slots beyond the capacity are dropped and flagged
 // (the reference writes past its 32-slot row).
-__global__ void __launch_bounds__(kThreads)
+//
+// A row of three cells along x is consecutive in the hash, so it is one
+// range of the cell table.  The nine ranges are read at once and then walked
+// as one sequence of candidates, the next candidate's position loaded before
+// the current one is tested, so a warp runs as long as its longest sequence
+// and not as the sum of the longest cells (32-lane divergence).  Rows and end
+// cells that no partner can reach are left out first (reach: the particle's
+// radius + the largest radius + the skin; the margin covers the rounding of
+// the cell coordinates and of the pair test): the reference's cells are two
+// largest radii wide, so a small sphere reaches few of its 27.
+constexpr int kNlistThreads = 128;
+__global__ void __launch_bounds__(kNlistThreads)
 k_nlist(const SimParams* __restrict__ P, const float4* __restrict__ pos, int n_max,
-        const uint32_t* __restrict__ cstart, const uint32_t* __restrict__ cend, NbrList nl,
-        StepCtl* ctl, const int* gate) {
+        const uint32_t* __restrict__ start, NbrList nl, StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
+  __shared__ uint2 row[9][kNlistThreads];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) ctl->epoch += 1;
   const int n = ctl->n_cur;
@@ -240,39 +250,65 @@ k_nlist(const SimParams* __restrict__ P, const float4* __restrict__ pos, int n_m
   // larger sphere of every pair checks that this fits in one cell edge
   if (skin > 0.0f && 2.0f * ra + skin > fminf(P->cell.x, fminf(P->cell.y, P->cell.z)))
     st |= kStatusCellTooSmall;
+  int rows = 0;
   if (in_grid(*P, g)) {
-    const int xs = g.x == 0 ? 0 : -1, xe = g.x == P->ncells.x - 1 ? 0 : 1;
-    const int ys = g.y == 0 ? 0 : -1, ye = g.y == P->ncells.y - 1 ? 0 : 1;
-    const int zs = g.z == 0 ? 0 : -1, ze = g.z == P->ncells.z - 1 ? 0 : 1;
-    for (int y = ys; y <= ye; ++y)
-      for (int z = zs; z <= ze; ++z)
-        for (int x = xs; x <= xe; ++x) {
-          const uint32_t h = grid_hash(*P, make_int3(g.x + x, g.y + y, g.z + z));
-          const uint32_t s = __ldg(cstart + h);
-          if (s == 0xffffffffu) continue;
-          const uint32_t e = __ldg(cend + h);
-          for (uint32_t j = s; j < e; ++j) {
-            if ((int)j == i) continue;
-            const float4 pb = __ldg(pos + j);
-            const float3 rel = pa - xyz(pb);
-            const float sr = ra + pb.w;
-            // skin 0: the reference's test, decided without the square root
-            // where that is exact (touches); with a skin the list need only
-            // hold every pair within it, so a bound a hair wider serves
-            bool keep;
-            if (skin > 0.0f) {
-              const float reach = sr + skin;
-              keep = dot3(rel, rel) < (reach * reach) * (1.0f + 0x1p-20f);
-            } else {
-              keep = touches(rel, sr);
-            }
-            if (keep) {
-              if (cnt < (uint32_t)nl.cap) nl.idx[(size_t)cnt * nl.stride + i] = j;
-              else st |= kStatusListOverflow;
-              ++cnt;
-            }
-          }
+    const float reach = (ra + P->r_max + skin) * (1.0f + 1e-5f);
+    const float lim = reach * reach;
+    const float2 dx = cell_gap(pa.x, P->origin.x, P->cell.x, g.x, P->ncells.x);
+    const float2 dy = cell_gap(pa.y, P->origin.y, P->cell.y, g.y, P->ncells.y);
+    const float2 dz = cell_gap(pa.z, P->origin.z, P->cell.z, g.z, P->ncells.z);
+#pragma unroll
+    for (int y = -1; y <= 1; ++y) {
+      const float gy = y < 0 ? dy.x : (y > 0 ? dy.y : 0.0f);
+      if (g.y + y < 0 || g.y + y >= P->ncells.y || gy * gy > lim) continue;
+#pragma unroll
+      for (int z = -1; z <= 1; ++z) {
+        const float gz = z < 0 ? dz.x : (z > 0 ? dz.y : 0.0f);
+        const float yz = gy * gy + gz * gz;
+        if (g.z + z < 0 || g.z + z >= P->ncells.z || yz > lim) continue;
+        const int xs = g.x == 0 || yz + dx.x * dx.x > lim ? 0 : -1;
+        const int xe = g.x == P->ncells.x - 1 || yz + dx.y * dx.y > lim ? 0 : 1;
+        const uint32_t h = grid_hash(*P, make_int3(g.x + xs, g.y + y, g.z + z));
+        const uint32_t s = __ldg(start + h), e = __ldg(start + h + (uint32_t)(xe - xs) + 1u);
+        if (s < e) row[rows++][threadIdx.x] = make_uint2(s, e);
+      }
+    }
+  }
+  if (rows > 0) {
+    uint2 q = row[0][threadIdx.x];
+    int r = 1;
+    uint32_t j = q.x;
+    float4 pn = __ldg(pos + j);
+    for (bool more = true; more;) {
+      const uint32_t jc = j;
+      const float4 pb = pn;
+      if (++j == q.y) {
+        more = r < rows;
+        if (more) {
+          q = row[r++][threadIdx.x];
+          j = q.x;
         }
+      }
+      if (more) pn = __ldg(pos + j);
+      if ((int)jc == i) continue;
+      const float3 rel = pa - xyz(pb);
+      const float sr = ra + pb.w;
+      // skin 0: the reference's test, decided without the square root
+      // where that is exact (touches); with a skin the list need only
+      // hold every pair within it, so a bound a hair wider serves
+      bool keep;
+      if (skin > 0.0f) {
+        const float reach = sr + skin;
+        keep = dot3(rel, rel) < (reach * reach) * (1.0f + 0x1p-20f);
+      } else {
+        keep = touches(rel, sr);
+      }
+      if (keep) {
+        if (cnt < (uint32_t)nl.cap) nl.idx[(size_t)cnt * nl.stride + i] = jc;
+        else st |= kStatusListOverflow;
+        ++cnt;
+      }
+    }
   }
   const uint32_t kept = cnt < (uint32_t)nl.cap ? cnt : (uint32_t)nl.cap;
   nl.cnt[i] = kept;
@@ -917,24 +953,21 @@ void launch_gate_graph(StepCtl* ctl, cudaGraphConditionalHandle h0, int* rb, int
 }
 
 void launch_hash(const SimParams* dp, const StateBuf& s, const OrderBuf& ob, int n_max,
-                 uint32_t* keys, StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_hash<<<blocks(n_max), kThreads, 0, st>>>(dp, s.pos, ob, n_max, keys, ctl, gate);
+                 const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st) {
+  k_hash<<<sort_blocks(n_max), kSortThreads, 0, st>>>(dp, s.pos, ob, n_max, cs, ctl, gate);
 }
 
 void launch_reorder(const StateBuf& src, const StateBuf& dst, const OrderBuf& ob, int n_max,
-                    const uint32_t* sorted_keys, const int32_t* perm, uint32_t* cell_start,
-                    uint32_t* cell_end, uint32_t ncell_tab, bool has_lift, int* flat_n,
-                    StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_reorder<<<blocks(n_max), kThreads, 0, st>>>(src, dst, ob, n_max, sorted_keys, perm, cell_start,
-                                                cell_end, ncell_tab, has_lift ? 1 : 0, flat_n,
-                                                ctl, gate);
+                    const CellSort& cs, bool has_lift, int* flat_n, StepCtl* ctl, const int* gate,
+                    cudaStream_t st) {
+  k_reorder<<<sort_blocks(n_max), kSortThreads, 0, st>>>(src, dst, ob, n_max, cs,
+                                                         has_lift ? 1 : 0, flat_n, ctl, gate);
 }
 
 void launch_nlist(const SimParams* dp, const StateBuf& s, int n_max, const uint32_t* cell_start,
-                  const uint32_t* cell_end, NbrList nl, StepCtl* ctl, const int* gate,
-                  cudaStream_t st) {
-  k_nlist<<<blocks(n_max), kThreads, 0, st>>>(dp, s.pos, n_max, cell_start, cell_end, nl, ctl,
-                                              gate);
+                  NbrList nl, StepCtl* ctl, const int* gate, cudaStream_t st) {
+  k_nlist<<<(n_max + kNlistThreads - 1) / kNlistThreads, kNlistThreads, 0, st>>>(
+      dp, s.pos, n_max, cell_start, nl, ctl, gate);
 }
 
 void launch_step(const SimParams* dp, const WallOp* ops, WallGrid wg, const StateBuf& in_plain,

@@ -1,6 +1,7 @@
 // dem_kernels.cuh -- launch interface of the per-step kernels.
 #pragma once
 
+#include "cell_sort.cuh"
 #include "dem_common.cuh"
 
 namespace blaze {
@@ -146,15 +147,14 @@ void launch_gate_body(StepCtl* ctl, cudaGraphConditionalHandle h0, cudaStream_t 
 void launch_gate_if(StepCtl* ctl, cudaGraphConditionalHandle h, float skin, float look,
                     int block_start, float vwall, cudaStream_t st);
 void launch_hash(const SimParams* dp, const StateBuf& s, const OrderBuf& ob, int n_max,
-                 uint32_t* keys, StepCtl* ctl, const int* gate, cudaStream_t st);
+                 const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st);
 // (flat_n, when given, is reset for the contact-list kernel's flat list)
 void launch_reorder(const StateBuf& src, const StateBuf& dst, const OrderBuf& ob, int n_max,
-                    const uint32_t* sorted_keys, const int32_t* perm, uint32_t* cell_start,
-                    uint32_t* cell_end, uint32_t ncell_tab, bool has_lift, int* flat_n,
-                    StepCtl* ctl, const int* gate, cudaStream_t st);
+                    const CellSort& cs, bool has_lift, int* flat_n, StepCtl* ctl, const int* gate,
+                    cudaStream_t st);
+// cell_start: the cell table of the sort (CellSort::start)
 void launch_nlist(const SimParams* dp, const StateBuf& s, int n_max, const uint32_t* cell_start,
-                  const uint32_t* cell_end, NbrList nl, StepCtl* ctl, const int* gate,
-                  cudaStream_t st);
+                  NbrList nl, StepCtl* ctl, const int* gate, cudaStream_t st);
 // eb: when not null, the step also writes each particle's energy-tally
 // values (particle-particle, volume objects, world objects; FP64) to
 // eb[c * n_max + i].  fast: the contracted particle-particle law (ignored

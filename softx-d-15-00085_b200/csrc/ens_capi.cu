@@ -15,7 +15,6 @@
 #include "ens_adjoint.cuh"
 #include "ens_kernels.cuh"
 #include "mix_kernels.cuh"
-#include "radix_sort.cuh"
 
 using namespace blaze;
 
@@ -52,12 +51,9 @@ struct blaze_ens {
   uint32_t* d_tri_off = nullptr;
   uint32_t* d_tri_ids = nullptr;
   uint32_t ncell_tab = 0;
-  int key_bits = 1;
   EnsBufs b{};
   int cur = 0;
-  RadixSortBuffers rs{};
-  uint32_t* cstart = nullptr;
-  uint32_t* cend = nullptr;
+  CellSort cs{};
   StepCtl* ctl = nullptr;
   StepCtl* h_ctl = nullptr;
   int* d_sys_of = nullptr;
@@ -339,9 +335,9 @@ void free_ens(blaze_ens* e) {
     f(e->b.pid[k]); f(e->b.wh[k]);
     f(e->b.L[k].idx); f(e->b.L[k].cnt); f(e->b.L[k].mask);
     f(e->b.L[k].hx); f(e->b.L[k].hy); f(e->b.L[k].hz); f(e->b.L[k].src);
-    f(e->rs.keys[k]); f(e->rs.vals[k]);
   }
-  f(e->rs.counts); f(e->rs.totals); f(e->cstart); f(e->cend); f(e->ctl); f(e->d_rb);
+  f(e->cs.key); f(e->cs.slot); f(e->cs.member); f(e->cs.perm); f(e->cs.cnt); f(e->cs.start);
+  f(e->cs.tile); f(e->cs.spec); f(e->ctl); f(e->d_rb);
   f(e->d_sys); f(e->d_walls); f(e->d_tri_off); f(e->d_tri_ids); f(e->d_sys_of);
   f(e->st_pos3); f(e->st_rad); f(e->st_vel3); f(e->st_avel3); f(e->st_sys); f(e->st_pid);
   f(e->d_flags); f(e->cap.f); f(e->cap.t); f(e->d_pw); f(e->d_rot);
@@ -400,26 +396,21 @@ int upload_params(blaze_ens* e) {
 int enqueue_rebuild(blaze_ens* e, const int* gate, cudaStream_t st) {
   const int n = e->n;
   const EnsGeom g = geom(e);
-  ens_launch_hash(g, e->b, e->cur, n, e->rs.keys[0], e->ctl, gate, st);
-  const int res = radix_sort_pairs(e->rs, n, e->key_bits, true, gate, st);
-  CK(cudaMemsetAsync(e->cstart, 0xff, sizeof(uint32_t) * e->ncell_tab, st));
-  ens_launch_reorder(e->b, e->cur, n, e->rs.keys[res], e->rs.vals[res], e->cstart, e->cend,
-                     e->ncell_tab, e->ctl, gate, st);
-  ens_launch_nlist(g, e->b, n, e->rs.vals[res], e->cstart, e->cend, e->ctl, gate, st);
+  ens_launch_hash(g, e->b, e->cur, n, e->cs, e->ctl, gate, st);
+  cell_scan_place(e->cs, n, &e->ctl->epoch, gate, st);
+  ens_launch_reorder(e->b, e->cur, n, e->cs, e->ctl, gate, st);
+  ens_launch_nlist(g, e->b, n, e->cs, e->ctl, gate, st);
   if (e->npoly > 0) {
-    mix_launch_plist(g, e->b, mix_bufs(e), e->cstart, e->cend, e->ctl, gate, st);
+    mix_launch_plist(g, e->b, mix_bufs(e), e->cs.start, e->ctl, gate, st);
     mix_launch_twins(e->b, mix_bufs(e), n, e->ctl, gate, st);
   }
-  ens_launch_epoch(e->ctl, gate, st);
   return 0;
 }
 
 int rebuild_kernel_count(const blaze_ens* e) {
-  return 4 + 3 * std::max(1, (e->key_bits + kRadixBits - 1) / kRadixBits) + (e->npoly > 0 ? 2 : 0);
+  return 3 + kCellSortKernels + (e->npoly > 0 ? 2 : 0);
 }
 
-// The step's kernels: polyhedron geometry, the sphere step, the polyhedron
-// step (the last two read the same input state and write disjoint entries).
 // The step's kernels: polyhedron geometry, the polyhedron step (which leaves
 // the sphere-polyhedron pairs' forces on the spheres), the sphere step; the
 // last two read the same input state and write disjoint entries.  ev
@@ -700,9 +691,6 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
       }
     }
   }
-  const uint32_t top = e->ncell_tab + 1u;
-  e->key_bits = 1;
-  while (e->key_bits < 32 && (top >> e->key_bits) != 0) e->key_bits++;
   CKF(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
   CKF(cudaStreamCreateWithFlags(&e->aux, cudaStreamNonBlocking));
   CKF(cudaStreamCreateWithFlags(&e->aux2, cudaStreamNonBlocking));
@@ -723,18 +711,23 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
     CKF(dalloc(&e->b.L[k].hy, (size_t)cap * n));
     CKF(dalloc(&e->b.L[k].hz, (size_t)cap * n));
     CKF(dalloc(&e->b.L[k].src, (size_t)cap * n));
-    CKF(dalloc(&e->rs.keys[k], n));
-    CKF(dalloc(&e->rs.vals[k], n));
     CKF(cudaMemset(e->b.L[k].cnt, 0, sizeof(uint32_t) * n));
     CKF(cudaMemset(e->b.L[k].mask, 0, sizeof(uint32_t) * n));
   }
-  const int tiles = (n + kTileKeys - 1) / kTileKeys;
-  e->rs.max_n = n;
-  e->rs.max_tiles = tiles;
-  CKF(dalloc(&e->rs.counts, (size_t)kRadixDigits * std::max(tiles, 1)));
-  CKF(dalloc(&e->rs.totals, kRadixDigits));
-  CKF(dalloc(&e->cstart, e->ncell_tab));
-  CKF(dalloc(&e->cend, e->ncell_tab));
+  {
+    const size_t tiles = cell_tiles(e->ncell_tab);
+    e->cs.ncell = e->ncell_tab;
+    CKF(dalloc(&e->cs.key, n));
+    CKF(dalloc(&e->cs.slot, n));
+    CKF(dalloc(&e->cs.member, n));
+    CKF(dalloc(&e->cs.perm, n));
+    CKF(dalloc(&e->cs.spec, (size_t)2 * sort_blocks(n)));
+    CKF(dalloc(&e->cs.cnt, tiles * kTileCells));
+    CKF(dalloc(&e->cs.start, tiles * kTileCells));
+    CKF(dalloc(&e->cs.tile, tiles + 1));
+    CKF(cudaMemset(e->cs.cnt, 0, sizeof(uint32_t) * tiles * kTileCells));
+    CKF(cudaMemset(e->cs.tile, 0, sizeof(uint32_t) * (tiles + 1)));
+  }
   CKF(dalloc(&e->ctl, 1));
   CKF(dalloc(&e->d_rb, kGraphSteps));
   CKF(cudaMemset(e->d_rb, 0, sizeof(int) * kGraphSteps));
@@ -1445,11 +1438,6 @@ struct blaze_ens_adj {
 
 namespace {
 
-int sort_result(const blaze_ens* e) {
-  const int passes = std::max(1, (e->key_bits + kRadixBits - 1) / kRadixBits);
-  return passes & 1;
-}
-
 void free_adj(blaze_ens_adj* a) {
   if (!a) return;
   for (cudaEvent_t ev : a->ev)
@@ -1528,7 +1516,6 @@ int restore_checkpoint(blaze_ens_adj* a, const EnsCheckpoint& c) {
 // re-sort), then the tape tick and the recording step.
 int build_record_graph(blaze_ens_adj* a, int c) {
   blaze_ens* e = a->e;
-  const int res = sort_result(e);
   const int saved = e->cur;
   e->cur = c;
   cudaGraph_t g = nullptr;
@@ -1560,7 +1547,7 @@ int build_record_graph(blaze_ens_adj* a, int c) {
                                      cudaStreamCaptureModeThreadLocal));
     CK(cudaMemsetAsync(e->d_rb + k, 0x01, sizeof(int), e->aux));
     int rc = enqueue_rebuild(e, nullptr, e->aux);
-    adj_launch_list(e->b, a->tape, e->n, e->ctl, nullptr, 1, e->rs.vals[res], e->aux);
+    adj_launch_list(e->b, a->tape, e->n, e->ctl, nullptr, 1, e->cs.perm, e->aux);
     cudaGraph_t tmp = nullptr;
     CK(cudaStreamEndCapture(e->aux, &tmp));
     if (rc) return rc;
@@ -1585,7 +1572,6 @@ int build_record_graph(blaze_ens_adj* a, int c) {
 int record_segment(blaze_ens_adj* a, int s, unsigned long long origin, unsigned long long lim,
                    TapeSeg& sg) {
   blaze_ens* e = a->e;
-  const int res = sort_result(e);
   const int slot0 = s * a->K, len = std::min(a->K, a->nsteps - slot0);
   cudaStream_t st = e->stream;
   adj_launch_seg_start(a->tape, slot0, len, origin, a->stride, lim, st);
@@ -1606,7 +1592,7 @@ int record_segment(blaze_ens_adj* a, int s, unsigned long long origin, unsigned 
     launch_gate(e->ctl, st);
     int rc = enqueue_rebuild(e, &e->ctl->rebuilt, st);
     if (rc) return rc;
-    adj_launch_list(e->b, a->tape, e->n, e->ctl, &e->ctl->rebuilt, 1, e->rs.vals[res], st);
+    adj_launch_list(e->b, a->tape, e->n, e->ctl, &e->ctl->rebuilt, 1, e->cs.perm, st);
     adj_launch_tick(a->tape, &e->ctl->rebuilt, st);
     ens_launch_step_record(geom(e), e->b, e->cur, e->n, e->ctl, StepLink{&e->ctl->rebuilt, 0, 0},
                            a->tape, e->opt.block, st);

@@ -1,11 +1,10 @@
 // ens_kernels.cu -- kernels of the ensemble path (see ens_kernels.cuh).
 //
 //   k_ens_hash     system-prefixed cell key per particle
-//   [radix sort, radix_sort.cu]
-//   k_ens_reorder  gather state, pid and wall history into sorted order + cell table
+//   [counting sort by cell and cell table, cell_sort.cu]
+//   k_ens_reorder  move state, pid and wall history into sorted order
 //   k_ens_nlist    27-cell Verlet list inside the particle's own system, carrying
 //                  the tangential history of every surviving contact by partner pid
-//   k_ens_epoch    one thread: the new list becomes current
 //   k_ens_step     pair law + walls + symplectic Euler, fused, gather only
 //
 // The contact model (per pair, with m* = ma mb / (ma + mb), R* = ra rb / (ra + rb),
@@ -34,36 +33,40 @@ namespace {
 constexpr int kThreads = 256;
 
 // ------------------------------------------------------------------- hash
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSortThreads)
 k_ens_hash(EnsGeom g, const float4* __restrict__ pos, const float4* __restrict__ vel, int n,
-           uint32_t* __restrict__ keys, StepCtl* ctl, const int* gate) {
+           CellSort cs, StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t sys = __float_as_uint(vel[i].w) & kSysMask;
-  const EnsSysDev& S = g.sys[sys];
-  const int3 c = ens_cell(S, xyz(pos[i]));
-  uint32_t st = 0, key;
-  if (ens_in(S, c)) {
-    key = ens_key(S, c);
-  } else {
-    key = g.ncell_tab;
-    st = kStatusOutOfGrid;
+  const int i = blockIdx.x * kSortThreads + threadIdx.x;
+  const bool valid = i < n;
+  uint32_t st = 0, key = 0;
+  if (valid) {
+    const uint32_t sys = __float_as_uint(vel[i].w) & kSysMask;
+    const EnsSysDev& S = g.sys[sys];
+    const int3 c = ens_cell(S, xyz(pos[i]));
+    if (ens_in(S, c)) {
+      key = ens_key(S, c);
+    } else {
+      key = g.ncell_tab;
+      st = kStatusOutOfGrid;
+    }
   }
-  keys[i] = key;
+  cell_count(cs, i, valid, key);
   ens_flag(ctl, st);
 }
 
 // ---------------------------------------------------------------- reorder
-__global__ void __launch_bounds__(kThreads)
-k_ens_reorder(StateBuf src, StateBuf dst, EnsBufs b, int n, const uint32_t* __restrict__ keys,
-              const int32_t* __restrict__ perm, uint32_t* __restrict__ cstart,
-              uint32_t* __restrict__ cend, uint32_t ncell_tab, StepCtl* ctl, const int* gate) {
+// (the place pass before it has already counted the re-sort: the old lists
+// are those of the other parity)
+__global__ void __launch_bounds__(kSortThreads)
+k_ens_reorder(StateBuf src, StateBuf dst, EnsBufs b, int n, CellSort cs, const StepCtl* ctl,
+              const int* gate) {
   if (gate && *gate == 0) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int e = ctl->epoch & 1;
-  const int j = perm[i];
+  const int j = blockIdx.x * kSortThreads + threadIdx.x;
+  const bool valid = j < n;
+  const int i = cell_dest(cs, j, valid);
+  if (!valid) return;
+  const int e = (ctl->epoch & 1) ^ 1;
   const float4 x = src.pos[j];
   dst.pos[i] = x;
   const float4 v = src.vel[j];
@@ -83,26 +86,27 @@ k_ens_reorder(StateBuf src, StateBuf dst, EnsBufs b, int n, const uint32_t* __re
     for (int q = 0; q < kWallSlots; ++q)
       b.wh[e ^ 1][(size_t)q * b.stride + i] = b.wh[e][(size_t)q * b.stride + j];
   }
-  const uint32_t k = keys[i];
-  if (k < ncell_tab) {
-    if (i == 0 || keys[i - 1] != k) cstart[k] = (uint32_t)i;
-    if (i == n - 1 || keys[i + 1] != k) cend[k] = (uint32_t)i + 1u;
-  }
 }
 
 // ------------------------------------------------------------------ nlist
 // Pairs with |xi - xj|^2 < (ri + rj + skin)^2 from the 27 surrounding cells
 // of the particle's own system (z, y, x order; j ascending inside a cell).
 // The history of a slot of the old list moves to the new slot of the same
-// partner (matched by pid).
-__global__ void __launch_bounds__(kThreads)
+// partner (matched by pid).  Rows of three cells are ranges of the cell
+// table, walked as one sequence of candidates with the next position loaded
+// ahead; rows and end cells out of reach are left out (see k_nlist): a
+// partner's radius is at most (cell - skin) / 2 (blaze_ens_set_state), so the
+// reach is ra + (cell + skin) / 2.
+constexpr int kNlistThreads = 128;
+__global__ void __launch_bounds__(kNlistThreads)
 k_ens_nlist(EnsGeom g, EnsBufs b, const float4* __restrict__ pos, const float4* __restrict__ vel,
-            int n, const int32_t* __restrict__ perm, const uint32_t* __restrict__ cstart,
-            const uint32_t* __restrict__ cend, StepCtl* ctl, const int* gate) {
+            int n, const int32_t* __restrict__ perm, const uint32_t* __restrict__ start,
+            StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
+  __shared__ uint2 row[9][kNlistThreads];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int e = ctl->epoch & 1;
+  const int e = (ctl->epoch & 1) ^ 1;
   const EnsList Lo = b.L[e], Ln = b.L[e ^ 1];
   const int* pid_old = b.pid[e];
   const int* pid_new = b.pid[e ^ 1];
@@ -122,65 +126,85 @@ k_ens_nlist(EnsGeom g, EnsBufs b, const float4* __restrict__ pos, const float4* 
   const uint32_t cnt_o = Lo.cnt[io];
   const uint32_t mask_o = Lo.mask[io];
   uint32_t cnt = 0, mask = 0, st = 0;
+  int rows = 0;
   if (ens_in(S, c)) {
-    const int x0 = c.x > 0 ? c.x - 1 : 0, x1 = c.x < S.nc.x - 1 ? c.x + 1 : c.x;
-    const int y0 = c.y > 0 ? c.y - 1 : 0, y1 = c.y < S.nc.y - 1 ? c.y + 1 : c.y;
-    const int z0 = c.z > 0 ? c.z - 1 : 0, z1 = c.z < S.nc.z - 1 ? c.z + 1 : c.z;
-    for (int z = z0; z <= z1; ++z)
-      for (int y = y0; y <= y1; ++y) {
-        const uint32_t row = S.cell_off + (uint32_t)(S.nc.x * (y + S.nc.y * z));
-        for (int x = x0; x <= x1; ++x) {
-          const uint32_t h = row + (uint32_t)x;
-          const uint32_t s = __ldg(cstart + h);
-          if (s == 0xffffffffu) continue;
-          const uint32_t eo = __ldg(cend + h);
-          for (uint32_t j = s; j < eo; ++j) {
-            if ((int)j == i) continue;
-            const float4 pb = __ldg(pos + j);
-            const float3 rel = pa - xyz(pb);
-            const float lim = (ra + fabsf(pb.w)) + g.skin;   // a polyhedron: its bounding radius
-            if (!(dot3(rel, rel) < lim * lim)) continue;
-            if (cnt < (uint32_t)b.cap) {
-              Ln.idx[cnt * stride + i] = j;
-              uint8_t from = 0xffu;
-              uint32_t mo = mask_o;
-              if (mo) {
-                const int pj = pid_new[j];
-                while (mo) {
-                  const int ko = __ffs(mo) - 1;
-                  mo &= mo - 1u;
-                  if ((uint32_t)ko >= cnt_o) break;
-                  const size_t so = (size_t)ko * stride + io;
-                  if (pid_old[Lo.idx[so]] == pj) {
-                    const size_t sn = (size_t)cnt * stride + i;
-                    Ln.hx[sn] = Lo.hx[so];
-                    Ln.hy[sn] = Lo.hy[so];
-                    Ln.hz[sn] = Lo.hz[so];
-                    mask |= 1u << cnt;
-                    from = (uint8_t)ko;
-                    break;
-                  }
-                }
-              }
-              if (Ln.src) Ln.src[cnt * stride + i] = from;
-            } else {
-              st |= kStatusListOverflow;
-            }
-            ++cnt;
-          }
-        }
+    const float reach = (ra + 0.5f * (S.cell + g.skin)) * (1.0f + 1e-5f);
+    const float lim = reach * reach;
+    const float2 dx = cell_gap(pa.x, S.origin.x, S.cell, c.x, S.nc.x);
+    const float2 dy = cell_gap(pa.y, S.origin.y, S.cell, c.y, S.nc.y);
+    const float2 dz = cell_gap(pa.z, S.origin.z, S.cell, c.z, S.nc.z);
+#pragma unroll
+    for (int z = -1; z <= 1; ++z) {
+      const float gz = z < 0 ? dz.x : (z > 0 ? dz.y : 0.0f);
+      if (c.z + z < 0 || c.z + z >= S.nc.z || gz * gz > lim) continue;
+#pragma unroll
+      for (int y = -1; y <= 1; ++y) {
+        const float gy = y < 0 ? dy.x : (y > 0 ? dy.y : 0.0f);
+        const float yz = gy * gy + gz * gz;
+        if (c.y + y < 0 || c.y + y >= S.nc.y || yz > lim) continue;
+        const int x0 = c.x == 0 || yz + dx.x * dx.x > lim ? c.x : c.x - 1;
+        const int x1 = c.x == S.nc.x - 1 || yz + dx.y * dx.y > lim ? c.x : c.x + 1;
+        const uint32_t h = S.cell_off + (uint32_t)(S.nc.x * (c.y + y + S.nc.y * (c.z + z)));
+        const uint32_t s0 = __ldg(start + h + (uint32_t)x0);
+        const uint32_t s1 = __ldg(start + h + (uint32_t)x1 + 1u);
+        if (s0 < s1) row[rows++][threadIdx.x] = make_uint2(s0, s1);
       }
+    }
   } else {
     st |= kStatusOutOfGrid;
+  }
+  if (rows > 0) {
+    uint2 q = row[0][threadIdx.x];
+    int r = 1;
+    uint32_t jn = q.x;
+    float4 pn = __ldg(pos + jn);
+    for (bool more = true; more;) {
+      const uint32_t j = jn;
+      const float4 pb = pn;
+      if (++jn == q.y) {
+        more = r < rows;
+        if (more) {
+          q = row[r++][threadIdx.x];
+          jn = q.x;
+        }
+      }
+      if (more) pn = __ldg(pos + jn);
+      if ((int)j == i) continue;
+      const float3 rel = pa - xyz(pb);
+      const float lim = (ra + fabsf(pb.w)) + g.skin;   // a polyhedron: its bounding radius
+      if (!(dot3(rel, rel) < lim * lim)) continue;
+      if (cnt < (uint32_t)b.cap) {
+        Ln.idx[cnt * stride + i] = j;
+        uint8_t from = 0xffu;
+        uint32_t mo = mask_o;
+        if (mo) {
+          const int pj = pid_new[j];
+          while (mo) {
+            const int ko = __ffs(mo) - 1;
+            mo &= mo - 1u;
+            if ((uint32_t)ko >= cnt_o) break;
+            const size_t so = (size_t)ko * stride + io;
+            if (pid_old[Lo.idx[so]] == pj) {
+              const size_t sn = (size_t)cnt * stride + i;
+              Ln.hx[sn] = Lo.hx[so];
+              Ln.hy[sn] = Lo.hy[so];
+              Ln.hz[sn] = Lo.hz[so];
+              mask |= 1u << cnt;
+              from = (uint8_t)ko;
+              break;
+            }
+          }
+        }
+        if (Ln.src) Ln.src[cnt * stride + i] = from;
+      } else {
+        st |= kStatusListOverflow;
+      }
+      ++cnt;
+    }
   }
   Ln.cnt[i] = cnt < (uint32_t)b.cap ? cnt : (uint32_t)b.cap;
   Ln.mask[i] = mask;
   ens_flag(ctl, st);
-}
-
-__global__ void k_ens_epoch(StepCtl* ctl, const int* gate) {
-  if (gate && *gate == 0) return;
-  ctl->epoch += 1;
 }
 
 // ------------------------------------------------------------------- step
@@ -851,27 +875,21 @@ inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
 
 }  // namespace
 
-void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, uint32_t* keys,
+void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, const CellSort& cs,
                      StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_ens_hash<<<nblk(n), kThreads, 0, st>>>(g, b.S[cur].pos, b.S[cur].vel, n, keys, ctl, gate);
+  k_ens_hash<<<sort_blocks(n), kSortThreads, 0, st>>>(g, b.S[cur].pos, b.S[cur].vel, n, cs, ctl,
+                                                      gate);
 }
 
-void ens_launch_reorder(const EnsBufs& b, int cur, int n, const uint32_t* keys,
-                        const int32_t* perm, uint32_t* cstart, uint32_t* cend, uint32_t ncell_tab,
-                        StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_ens_reorder<<<nblk(n), kThreads, 0, st>>>(b.S[cur], b.S[2], b, n, keys, perm, cstart, cend,
-                                              ncell_tab, ctl, gate);
+void ens_launch_reorder(const EnsBufs& b, int cur, int n, const CellSort& cs, StepCtl* ctl,
+                        const int* gate, cudaStream_t st) {
+  k_ens_reorder<<<sort_blocks(n), kSortThreads, 0, st>>>(b.S[cur], b.S[2], b, n, cs, ctl, gate);
 }
 
-void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const int32_t* perm,
-                      const uint32_t* cstart, const uint32_t* cend, StepCtl* ctl,
+void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const CellSort& cs, StepCtl* ctl,
                       const int* gate, cudaStream_t st) {
-  k_ens_nlist<<<nblk(n), kThreads, 0, st>>>(g, b, b.S[2].pos, b.S[2].vel, n, perm, cstart, cend,
-                                            ctl, gate);
-}
-
-void ens_launch_epoch(StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_ens_epoch<<<1, 1, 0, st>>>(ctl, gate);
+  k_ens_nlist<<<(n + kNlistThreads - 1) / kNlistThreads, kNlistThreads, 0, st>>>(
+      g, b, b.S[2].pos, b.S[2].vel, n, cs.perm, cs.start, ctl, gate);
 }
 
 void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl* ctl,

@@ -294,15 +294,14 @@ __device__ __forceinline__ uint32_t tape_reserve(uint32_t words, unsigned long l
   return (uint32_t)(s_start - base) + s_warp[w] + (x - words);
 }
 
-void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, uint32_t* keys,
+// One re-sort: hash (key and count), cell_scan_place on &ctl->epoch, reorder,
+// nlist.
+void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, const CellSort& cs,
                      StepCtl* ctl, const int* gate, cudaStream_t st);
-void ens_launch_reorder(const EnsBufs& b, int cur, int n, const uint32_t* keys,
-                        const int32_t* perm, uint32_t* cstart, uint32_t* cend, uint32_t ncell_tab,
-                        StepCtl* ctl, const int* gate, cudaStream_t st);
-void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const int32_t* perm,
-                      const uint32_t* cstart, const uint32_t* cend, StepCtl* ctl,
+void ens_launch_reorder(const EnsBufs& b, int cur, int n, const CellSort& cs, StepCtl* ctl,
+                        const int* gate, cudaStream_t st);
+void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const CellSort& cs, StepCtl* ctl,
                       const int* gate, cudaStream_t st);
-void ens_launch_epoch(StepCtl* ctl, const int* gate, cudaStream_t st);
 // `block`: threads per block (64 .. kMaxStepBlock, a multiple of 32).
 constexpr int kMaxStepBlock = 512;
 void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl* ctl,

@@ -67,17 +67,17 @@ k_mix_geom(MixBufs m) {
 // Pairs with |xi - xj|^2 < (ri + rj + skin)^2 (bounding radii) from the 27
 // surrounding cells, in the sphere list's order (z, y, x; j ascending); the
 // history of an old slot moves to the new slot of the same partner pid.  A
-// warp per polyhedron: the lanes take consecutive candidates of a cell and
+// warp per polyhedron: the lanes take consecutive candidates of a row and
 // a ballot hands out the slots in candidate order.
 __global__ void __launch_bounds__(kThreads)
 k_mix_plist(EnsGeom g, EnsBufs b, MixBufs m, const float4* __restrict__ pos,
-            const float4* __restrict__ vel, const uint32_t* __restrict__ cstart,
-            const uint32_t* __restrict__ cend, StepCtl* ctl, const int* gate) {
+            const float4* __restrict__ vel, const uint32_t* __restrict__ start, StepCtl* ctl,
+            const int* gate) {
   if (gate && *gate == 0) return;
   const int lane = threadIdx.x & 31;
   const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (p >= m.npoly) return;
-  const int e = ctl->epoch & 1;
+  const int e = (ctl->epoch & 1) ^ 1;   // the lists before this re-sort
   const MixList Lo = m.L[e], Ln = m.L[e ^ 1];
   const int* pid_old = b.pid[e];
   const int* pid_new = b.pid[e ^ 1];
@@ -101,50 +101,47 @@ k_mix_plist(EnsGeom g, EnsBufs b, MixBufs m, const float4* __restrict__ pos,
     for (int z = z0; z <= z1; ++z)
       for (int y = y0; y <= y1; ++y) {
         const uint32_t row = S.cell_off + (uint32_t)(S.nc.x * (y + S.nc.y * z));
-        for (int x = x0; x <= x1; ++x) {
-          const uint32_t h = row + (uint32_t)x;
-          const uint32_t s0 = __ldg(cstart + h);
-          if (s0 == 0xffffffffu) continue;
-          const uint32_t eo = __ldg(cend + h);
-          for (uint32_t j0 = s0; j0 < eo; j0 += 32) {
-            const uint32_t j = j0 + (uint32_t)lane;
-            bool hit = false;
-            if (j < eo && (int)j != i) {
-              const float4 pb = __ldg(pos + j);
-              const float3 rel = pa - xyz(pb);
-              const float lim = (ra + fabsf(pb.w)) + g.skin;
-              hit = dot3(rel, rel) < lim * lim;
-            }
-            const uint32_t hb = __ballot_sync(0xffffffffu, hit);
-            if (hit) {
-              const uint32_t k = cnt + (uint32_t)__popc(hb & ((1u << lane) - 1u));
-              if (k < (uint32_t)kMixSlots) {
-                Ln.idx[(size_t)k * P + p] = j;
-                Ln.sep[(size_t)k * P + p] = -1;
-                unsigned long long mo = mask_o;
-                if (mo) {
-                  const int pj = pid_new[j];
-                  while (mo) {
-                    const int ko = __ffsll((long long)mo) - 1;
-                    mo &= mo - 1ull;
-                    if ((uint32_t)ko >= cnt_o) break;
-                    const size_t so = (size_t)ko * P + p;
-                    if (pid_old[Lo.idx[so]] == pj) {
-                      const size_t sn = (size_t)k * P + p;
-                      Ln.hx[sn] = Lo.hx[so];
-                      Ln.hy[sn] = Lo.hy[so];
-                      Ln.hz[sn] = Lo.hz[so];
-                      mask |= 1ull << k;
-                      break;
-                    }
+        // the row's cells are one range of the cell table
+        const uint32_t s0 = __ldg(start + row + (uint32_t)x0);
+        const uint32_t eo = __ldg(start + row + (uint32_t)x1 + 1u);
+        for (uint32_t j0 = s0; j0 < eo; j0 += 32) {
+          const uint32_t j = j0 + (uint32_t)lane;
+          bool hit = false;
+          if (j < eo && (int)j != i) {
+            const float4 pb = __ldg(pos + j);
+            const float3 rel = pa - xyz(pb);
+            const float lim = (ra + fabsf(pb.w)) + g.skin;
+            hit = dot3(rel, rel) < lim * lim;
+          }
+          const uint32_t hb = __ballot_sync(0xffffffffu, hit);
+          if (hit) {
+            const uint32_t k = cnt + (uint32_t)__popc(hb & ((1u << lane) - 1u));
+            if (k < (uint32_t)kMixSlots) {
+              Ln.idx[(size_t)k * P + p] = j;
+              Ln.sep[(size_t)k * P + p] = -1;
+              unsigned long long mo = mask_o;
+              if (mo) {
+                const int pj = pid_new[j];
+                while (mo) {
+                  const int ko = __ffsll((long long)mo) - 1;
+                  mo &= mo - 1ull;
+                  if ((uint32_t)ko >= cnt_o) break;
+                  const size_t so = (size_t)ko * P + p;
+                  if (pid_old[Lo.idx[so]] == pj) {
+                    const size_t sn = (size_t)k * P + p;
+                    Ln.hx[sn] = Lo.hx[so];
+                    Ln.hy[sn] = Lo.hy[so];
+                    Ln.hz[sn] = Lo.hz[so];
+                    mask |= 1ull << k;
+                    break;
                   }
                 }
-              } else {
-                st |= kStatusListOverflow;
               }
+            } else {
+              st |= kStatusListOverflow;
             }
-            cnt += (uint32_t)__popc(hb);
           }
+          cnt += (uint32_t)__popc(hb);
         }
       }
   } else {
@@ -163,7 +160,7 @@ k_mix_plist(EnsGeom g, EnsBufs b, MixBufs m, const float4* __restrict__ pos,
 }
 
 // The twin of every sphere slot that holds a polyhedron: the polyhedron's
-// slot that holds the sphere (new lists, before the epoch turns).
+// slot that holds the sphere (new lists).
 __global__ void __launch_bounds__(kThreads)
 k_mix_twins(EnsBufs b, MixBufs m, const float4* __restrict__ pos,
             const float4* __restrict__ angv, int n, StepCtl* ctl, const int* gate) {
@@ -171,7 +168,7 @@ k_mix_twins(EnsBufs b, MixBufs m, const float4* __restrict__ pos,
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   if (pos[i].w < 0.0f) return;
-  const int e = ctl->epoch & 1;
+  const int e = (ctl->epoch & 1) ^ 1;   // the lists before this re-sort
   const EnsList Ln = b.L[e ^ 1];
   const MixList Pn = m.L[e ^ 1];
   const size_t stride = (size_t)b.stride, P = (size_t)m.npoly;
@@ -726,11 +723,10 @@ void mix_launch_geom(const MixBufs& m, cudaStream_t st) {
 }
 
 void mix_launch_plist(const EnsGeom& g, const EnsBufs& b, const MixBufs& m,
-                      const uint32_t* cstart, const uint32_t* cend, StepCtl* ctl,
-                      const int* gate, cudaStream_t st) {
+                      const uint32_t* start, StepCtl* ctl, const int* gate, cudaStream_t st) {
   if (m.npoly <= 0) return;
-  k_mix_plist<<<nblk(32 * m.npoly), kThreads, 0, st>>>(g, b, m, b.S[2].pos, b.S[2].vel, cstart,
-                                                       cend, ctl, gate);
+  k_mix_plist<<<nblk(32 * m.npoly), kThreads, 0, st>>>(g, b, m, b.S[2].pos, b.S[2].vel, start,
+                                                       ctl, gate);
 }
 
 void mix_launch_twins(const EnsBufs& b, const MixBufs& m, int n, StepCtl* ctl, const int* gate,

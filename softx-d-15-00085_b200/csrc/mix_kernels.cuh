@@ -30,7 +30,7 @@ void mix_launch_mark(const EnsBufs& b, int cur, const MixBufs& m, const int* cal
                      const float4* quat, cudaStream_t st);
 void mix_launch_geom(const MixBufs& m, cudaStream_t st);
 void mix_launch_plist(const EnsGeom& g, const EnsBufs& b, const MixBufs& m,
-                      const uint32_t* cstart, const uint32_t* cend, StepCtl* ctl,
+                      const uint32_t* start, StepCtl* ctl,
                       const int* gate, cudaStream_t st);
 // After k_mix_plist: per sphere slot holding a polyhedron, the polyhedron's
 // slot that holds the sphere.

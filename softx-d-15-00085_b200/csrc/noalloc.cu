@@ -1,5 +1,5 @@
 // noalloc.cu -- blaze_contact_list_static: the broad phase of the step (cell
-// keys, stable radix sort, cell table, contact list) for callers that cannot
+// keys, stable counting sort, cell table, contact list) for callers that cannot
 // allocate device memory.
 //
 // Who needs it: a host code that calls the broad phase between its own
@@ -26,11 +26,11 @@
 // results: serialise them.
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <mutex>
 
 #include "blaze_dem.h"
 #include "dem_kernels.cuh"
-#include "radix_sort.cuh"
 
 using namespace blaze;
 
@@ -39,26 +39,25 @@ namespace {
 constexpr int kMaxParticles = 65536;
 constexpr uint32_t kMaxCells = 262144;
 constexpr int kMaxDevices = 64;
-constexpr int kMaxTilesStatic = (kMaxParticles + kTileKeys - 1) / kTileKeys;
+constexpr size_t kCellWords = (size_t)cell_tiles(kMaxCells) * kTileCells;
 
 constexpr size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // Byte offsets of the pieces inside the scratch array.
 constexpr size_t kOffParams = 0;
 constexpr size_t kOffCtl = up256(kOffParams + sizeof(SimParams));
-constexpr size_t kOffKeys0 = up256(kOffCtl + sizeof(StepCtl));
-constexpr size_t kOffKeys1 = up256(kOffKeys0 + sizeof(uint32_t) * kMaxParticles);
-constexpr size_t kOffVals0 = up256(kOffKeys1 + sizeof(uint32_t) * kMaxParticles);
-constexpr size_t kOffVals1 = up256(kOffVals0 + sizeof(int32_t) * kMaxParticles);
-constexpr size_t kOffCounts = up256(kOffVals1 + sizeof(int32_t) * kMaxParticles);
-constexpr size_t kOffTotals = up256(kOffCounts + sizeof(uint32_t) * kRadixDigits * kMaxTilesStatic);
-constexpr size_t kOffPid0 = up256(kOffTotals + sizeof(uint32_t) * kRadixDigits);
+constexpr size_t kOffKey = up256(kOffCtl + sizeof(StepCtl));
+constexpr size_t kOffSlot = up256(kOffKey + sizeof(uint32_t) * kMaxParticles);
+constexpr size_t kOffMember = up256(kOffSlot + sizeof(uint32_t) * kMaxParticles);
+constexpr size_t kOffSpec = up256(kOffMember + sizeof(int32_t) * kMaxParticles);
+constexpr size_t kOffTile = up256(kOffSpec + sizeof(uint32_t) * 2 * sort_blocks(kMaxParticles));
+constexpr size_t kOffPid0 = up256(kOffTile + sizeof(uint32_t) * (cell_tiles(kMaxCells) + 1));
 constexpr size_t kOffPid1 = up256(kOffPid0 + sizeof(int) * kMaxParticles);
 constexpr size_t kOffSorted = up256(kOffPid1 + sizeof(int) * kMaxParticles);
 constexpr size_t kOffSpare = up256(kOffSorted + sizeof(float4) * kMaxParticles);
-constexpr size_t kOffCstart = up256(kOffSpare + sizeof(float4) * kMaxParticles);
-constexpr size_t kOffCend = up256(kOffCstart + sizeof(uint32_t) * kMaxCells);
-constexpr size_t kScratchBytes = up256(kOffCend + sizeof(uint32_t) * kMaxCells);
+constexpr size_t kOffCnt = up256(kOffSpare + sizeof(float4) * kMaxParticles);
+constexpr size_t kOffStart = up256(kOffCnt + sizeof(uint32_t) * kCellWords);
+constexpr size_t kScratchBytes = up256(kOffStart + sizeof(uint32_t) * kCellWords);
 
 static __device__ __align__(256) unsigned char g_scratch[kScratchBytes];
 
@@ -72,7 +71,7 @@ struct StaticParams {
   float3 origin, cell;
   int3 ncells;
   uint32_t ncell_tab;
-  float skin;
+  float skin, r_max;
   int max_nbr;
   int n;
 };
@@ -93,6 +92,7 @@ __global__ void k_static_init(StaticParams sp, SimParams* dp, StepCtl* ctl) {
   dp->ncells = sp.ncells;
   dp->ncell_tab = sp.ncell_tab;
   dp->skin = sp.skin;
+  dp->r_max = sp.r_max;
   dp->max_nbr = sp.max_nbr;
   ctl->n_cur = sp.n;
 }
@@ -151,25 +151,25 @@ extern "C" int blaze_contact_list_static(const float* pos4, int n, const Simulat
   sp.ncells = si->num_NNCells;
   sp.ncell_tab = (uint32_t)ntab;
   sp.skin = skin;
+  sp.r_max = std::numeric_limits<float>::infinity();   // the caller's radii are any
   sp.max_nbr = max_nbr;
   sp.n = n;
 
   SimParams* dp = reinterpret_cast<SimParams*>(base + kOffParams);
   StepCtl* ctl = reinterpret_cast<StepCtl*>(base + kOffCtl);
-  RadixSortBuffers rs;
-  rs.keys[0] = reinterpret_cast<uint32_t*>(base + kOffKeys0);
-  rs.keys[1] = reinterpret_cast<uint32_t*>(base + kOffKeys1);
-  rs.vals[0] = reinterpret_cast<int32_t*>(base + kOffVals0);
-  rs.vals[1] = reinterpret_cast<int32_t*>(base + kOffVals1);
-  rs.counts = reinterpret_cast<uint32_t*>(base + kOffCounts);
-  rs.totals = reinterpret_cast<uint32_t*>(base + kOffTotals);
-  rs.max_n = kMaxParticles;
-  rs.max_tiles = kMaxTilesStatic;
+  CellSort cs;
+  cs.key = reinterpret_cast<uint32_t*>(base + kOffKey);
+  cs.slot = reinterpret_cast<uint32_t*>(base + kOffSlot);
+  cs.member = reinterpret_cast<int32_t*>(base + kOffMember);
+  cs.perm = perm;
+  cs.cnt = reinterpret_cast<uint32_t*>(base + kOffCnt);
+  cs.start = reinterpret_cast<uint32_t*>(base + kOffStart);
+  cs.tile = reinterpret_cast<uint32_t*>(base + kOffTile);
+  cs.spec = reinterpret_cast<uint32_t*>(base + kOffSpec);
+  cs.ncell = (uint32_t)ntab;
   OrderBuf ob{};
   ob.pid[0] = reinterpret_cast<int*>(base + kOffPid0);
   ob.pid[1] = reinterpret_cast<int*>(base + kOffPid1);
-  uint32_t* cstart = reinterpret_cast<uint32_t*>(base + kOffCstart);
-  uint32_t* cend = reinterpret_cast<uint32_t*>(base + kOffCend);
   float4* in4 = const_cast<float4*>(reinterpret_cast<const float4*>(pos4));
   float4* sorted = reinterpret_cast<float4*>(base + kOffSorted);
   float4* spare = reinterpret_cast<float4*>(base + kOffSpare);
@@ -177,10 +177,6 @@ extern "C" int blaze_contact_list_static(const float* pos4, int n, const Simulat
   // it reads the positions twice and writes both copies into one spare buffer
   const StateBuf src{in4, in4, in4};
   const StateBuf dst{sorted, spare, spare};
-
-  int bits = 1;
-  const uint32_t top = (uint32_t)ntab + 1u;
-  while (bits < 32 && (top >> bits) != 0) bits++;
 
 #define CKS(x)                                    \
   do {                                            \
@@ -190,11 +186,11 @@ extern "C" int blaze_contact_list_static(const float* pos4, int n, const Simulat
   // what this call relies on starting from a known value
   k_static_init<<<1, 256, 0, st>>>(sp, dp, ctl);
   CKS(cudaMemsetAsync(ob.pid[0], 0, sizeof(int) * n, st));  // every particle live
-  CKS(cudaMemsetAsync(cstart, 0xff, sizeof(uint32_t) * ntab, st));
-  launch_hash(dp, src, ob, n, rs.keys[0], ctl, nullptr, st);
-  const int res = radix_sort_pairs(rs, n, bits, true, nullptr, st);
-  launch_reorder(src, dst, ob, n, rs.keys[res], rs.vals[res], cstart, cend, (uint32_t)ntab,
-                 false, nullptr, ctl, nullptr, st);
+  CKS(cudaMemsetAsync(cs.cnt, 0, sizeof(uint32_t) * (size_t)cell_tiles(cs.ncell) * kTileCells, st));
+  CKS(cudaMemsetAsync(cs.tile, 0, sizeof(uint32_t) * (cell_tiles(cs.ncell) + 1), st));
+  launch_hash(dp, src, ob, n, cs, ctl, nullptr, st);
+  cell_scan_place(cs, n, nullptr, nullptr, st);
+  launch_reorder(src, dst, ob, n, cs, false, nullptr, ctl, nullptr, st);
   NbrList nl;
   nl.idx = list;
   nl.cnt = nn;
@@ -202,8 +198,7 @@ extern "C" int blaze_contact_list_static(const float* pos4, int n, const Simulat
   nl.cap = max_nbr;
   nl.flat = nullptr;
   nl.flat_n = nullptr;
-  launch_nlist(dp, dst, n, cstart, cend, nl, ctl, nullptr, st);
-  CKS(cudaMemcpyAsync(perm, rs.vals[res], sizeof(int) * n, cudaMemcpyDeviceToDevice, st));
+  launch_nlist(dp, dst, n, cs.start, nl, ctl, nullptr, st);
   if (status)
     CKS(cudaMemcpyAsync(status, &ctl->status, sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
   CKS(cudaGetLastError());
