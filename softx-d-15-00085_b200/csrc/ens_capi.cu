@@ -50,6 +50,8 @@ struct blaze_ens {
   EnsWallDev* d_walls = nullptr;
   uint32_t* d_tri_off = nullptr;
   uint32_t* d_tri_ids = nullptr;
+  float4* d_tri_b = nullptr;
+  bool curved = false;        // some wall is a cylinder or a triangle
   uint32_t ncell_tab = 0;
   EnsBufs b{};
   int cur = 0;
@@ -108,6 +110,7 @@ struct blaze_ens {
   bool sgrid = false;
   uint32_t* d_stri_off = nullptr;
   uint32_t* d_stri_ids = nullptr;
+  float4* d_stri_b = nullptr;
   MixList ml[2] = {};
   // blaze_ens_set_profile: plain steps timed by phase
   bool prof = false;
@@ -126,13 +129,13 @@ EnsGeom geom(const blaze_ens* e) {
   g.tri_ids = e->d_tri_ids;
   g.stri_off = e->sgrid ? e->d_stri_off : e->d_tri_off;
   g.stri_ids = e->sgrid ? e->d_stri_ids : e->d_tri_ids;
+  g.tri_b = e->d_tri_b;
+  g.stri_b = e->sgrid ? e->d_stri_b : e->d_tri_b;
   g.ncell_tab = e->ncell_tab;
   g.law = e->opt.law;
   g.dt = e->opt.dt;
   g.skin = e->opt.skin;
-  g.curved = 0;
-  for (const EnsWallDev& w : e->hwalls)
-    if (w.kind != kWallPlane) g.curved = 1;
+  g.curved = e->curved ? 1 : 0;
   g.rot = e->d_rot;
   g.any_rot = e->any_rot ? 1 : 0;
   g.mix = MixView{};
@@ -317,6 +320,51 @@ void build_tri_lists(const blaze_ens* e, std::vector<uint32_t>& off, std::vector
   for (size_t c = 0; c < ntab; ++c) off[c + 1] += off[c];
 }
 
+// A sphere around triangle W: about the middle of its longest edge or its
+// centroid, whichever gives the smaller one, with the radius rounded up by
+// 1e-5 of the coordinates' size (the FP32 distance tests round at 1e-7).
+float4 tri_bound(const EnsWallDev& W) {
+  const double v[3][3] = {{W.a.x, W.a.y, W.a.z}, {W.b.x, W.b.y, W.b.z}, {W.c.x, W.c.y, W.c.z}};
+  auto dist = [](const double* p, const double* q) {
+    return std::sqrt((p[0] - q[0]) * (p[0] - q[0]) + (p[1] - q[1]) * (p[1] - q[1]) +
+                     (p[2] - q[2]) * (p[2] - q[2]));
+  };
+  int a = 0, b = 1;
+  for (int k = 0; k < 3; ++k)
+    if (dist(v[k], v[(k + 1) % 3]) > dist(v[a], v[b])) {
+      a = k;
+      b = (k + 1) % 3;
+    }
+  double mid[3], cen[3], size = 0.0;
+  for (int c = 0; c < 3; ++c) {
+    mid[c] = 0.5 * (v[a][c] + v[b][c]);
+    cen[c] = (v[0][c] + v[1][c] + v[2][c]) / 3.0;
+    for (int k = 0; k < 3; ++k) size = std::max(size, std::fabs(v[k][c]));
+  }
+  double rm = 0.0, rc = 0.0;
+  for (int k = 0; k < 3; ++k) {
+    rm = std::max(rm, dist(mid, v[k]));
+    rc = std::max(rc, dist(cen, v[k]));
+  }
+  const double* o = rm <= rc ? mid : cen;
+  const double r = std::min(rm, rc);
+  return make_float4((float)o[0], (float)o[1], (float)o[2],
+                     (float)((r + 1e-5 * (size + r)) * (1.0 + 1e-5)));
+}
+
+// The bounding spheres of a candidate list, uploaded.
+int upload_bounds(const blaze_ens* e, const std::vector<uint32_t>& ids, float4** d) {
+  std::vector<float4> one(e->hwalls.size()), bs(ids.size());
+  for (size_t w = 0; w < one.size(); ++w)
+    if (e->hwalls[w].kind == kWallTriangle) one[w] = tri_bound(e->hwalls[w]);
+  for (size_t k = 0; k < ids.size(); ++k) bs[k] = one[ids[k]];
+  if (*d) CK(cudaFree(*d));
+  *d = nullptr;
+  CK(dalloc(d, bs.size()));
+  if (!bs.empty()) CK(cudaMemcpy(*d, bs.data(), sizeof(float4) * bs.size(), cudaMemcpyHostToDevice));
+  return 0;
+}
+
 void drop_graphs(blaze_ens* e) {
   for (int c = 0; c < 2; ++c) {
     if (e->graph[c]) cudaGraphExecDestroy(e->graph[c]);
@@ -344,7 +392,7 @@ void free_ens(blaze_ens* e) {
   f(e->d_shapes); f(e->d_bv); f(e->d_bn); f(e->d_faces); f(e->d_edges); f(e->d_shape_of);
   f(e->d_pidx); f(e->d_quat); f(e->d_quat0); f(e->d_pat); f(e->d_ppath); f(e->d_gv); f(e->d_gf);
   f(e->d_pwh); f(e->d_pwn); f(e->d_psf); f(e->d_pst); f(e->d_twin);
-  f(e->d_stri_off); f(e->d_stri_ids);
+  f(e->d_stri_off); f(e->d_stri_ids); f(e->d_tri_b); f(e->d_stri_b);
   for (int k = 0; k < 2; ++k) {
     f(e->ml[k].idx); f(e->ml[k].cnt); f(e->ml[k].mlo); f(e->ml[k].mhi);
     f(e->ml[k].hx); f(e->ml[k].hy); f(e->ml[k].hz); f(e->ml[k].sep);
@@ -669,7 +717,10 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
   e->nwalls = nwalls;
   e->sys.assign(systems, systems + nsys);
   e->ncell_tab = (uint32_t)cells;
-  for (int w = 0; w < nwalls; ++w) e->hwalls.push_back(wall_dev(walls[w]));
+  for (int w = 0; w < nwalls; ++w) {
+    e->hwalls.push_back(wall_dev(walls[w]));
+    e->curved = e->curved || walls[w].kind != BLAZE_WALL_PLANE;
+  }
   // walls that turn in place with a drum: cylinders coaxial with it, planes
   // normal to its axis (their surfaces move; their positions do not)
   for (int s = 0; s < nsys; ++s) {
@@ -784,6 +835,8 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
     CKF(cudaMemcpy(e->d_tri_off, off.data(), sizeof(uint32_t) * off.size(), cudaMemcpyHostToDevice));
     if (!ids.empty())
       CKF(cudaMemcpy(e->d_tri_ids, ids.data(), sizeof(uint32_t) * ids.size(), cudaMemcpyHostToDevice));
+    rc = upload_bounds(e, ids, &e->d_tri_b);
+    if (rc) return fail(rc);
   }
   std::memset(e->h_ctl, 0, sizeof(StepCtl));
   e->h_ctl->n_cur = n;
@@ -1322,6 +1375,7 @@ int blaze_ens_set_polyhedra(blaze_ens* e, const blaze_shape* shapes, int nshapes
       if (!ids.empty())
         CK(cudaMemcpy(e->d_stri_ids, ids.data(), sizeof(uint32_t) * ids.size(),
                       cudaMemcpyHostToDevice));
+      if ((rc = upload_bounds(e, ids, &e->d_stri_b))) return rc;
     }
     e->sgrid = any;
     if ((rc = upload_params(e))) return rc;

@@ -685,6 +685,12 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     float best_d = 0.0f;
     bool face = false;
     for (uint32_t q = o0; q < o1; ++q) {
+      // most of a cell's triangles are out of reach: a sphere around each
+      // tells (rounded up by more than the test's own rounding, tri_bound)
+      const float4 bs = __ldg(g.stri_b + q);
+      const float3 dc = pd - xyz(bs);
+      const float reach = bs.w + ra;
+      if (dot3(dc, dc) > reach * reach) continue;
       const int id = (int)__ldg(g.stri_ids + q);
       float3 nrm;
       float delta;

@@ -153,8 +153,10 @@ struct EnsGeom {
   const EnsWallDev* walls;
   const uint32_t* tri_off;   // per global cell: candidate triangles (CSR), or null
   const uint32_t* tri_ids;
+  const float4* tri_b;       // per entry of tri_ids: a sphere (centre, radius) around the triangle
   const uint32_t* stri_off;  // the same on the spheres' grid (EnsSysDev::scell)
   const uint32_t* stri_ids;
+  const float4* stri_b;
   uint32_t ncell_tab;        // total hash-table entries
   int law;
   float dt, skin;

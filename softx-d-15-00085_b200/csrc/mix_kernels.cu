@@ -7,7 +7,8 @@ namespace blaze {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMixWarps = 4;      // warps (polyhedra) per block of the step
+constexpr int kMixWarps = 4;      // warps per polyhedron in the step
+constexpr int kMixBlock = 32 * kMixWarps;
 constexpr int kMixHits = 32;      // touching triangles kept per polyhedron and step
 
 inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
@@ -341,11 +342,23 @@ struct MixSmem {
   float4 t[kMixSlots];
   double4 v[kMixMaxV];      // geometry in the drum's frame (a turning drum)
   double4 fn[kMixMaxF];
-  double3 nd[kMixHits];     // touching triangles: unrounded normal, contact, id
-  MixHit hit[kMixHits];
-  int hid[kMixHits];
-  int hkind[kMixHits];      // 0: the triangle's face; 1, 2: a face of the polyhedron, an edge pair
+  uint32_t polys[2];        // slots whose polyhedron's bounding sphere overlaps
+  uint32_t touch[2];        // slots in contact
+  uint32_t nearby[kMixWarps];  // of a window of kMixBlock candidate triangles
+  int task;                 // next task of the window
+  // the window's nearby triangles, in ascending order
+  double3 nd[kMixBlock];    // unrounded normal
+  MixHit hit[kMixBlock];
+  int id[kMixBlock];
+  int kind[kMixBlock];      // 0: the triangle's face; 1, 2: a face of the polyhedron, an edge
+                            // pair; -1: apart
+  // the touching triangles
+  double3 knd[kMixHits];
+  MixHit khit[kMixHits];
+  int kid[kMixHits];
+  int kkind[kMixHits];
   float4 oh[kMixWallSlots]; // the polyhedron's wall histories before the step
+  float4 wf[32], wt[32];    // wall contacts' force and torque
 };
 
 __device__ __forceinline__ float3 mat_vec_f(const float* R, float3 v) {
@@ -357,18 +370,24 @@ __device__ __forceinline__ float3 mat_tvec_f(const float* R, float3 v) {
             (R[2] * v.x + R[5] * v.y) + R[8] * v.z);
 }
 
-// One warp per polyhedron.  The polyhedron's own force is summed by lane 0
-// in slot order, then the walls (planes in order, then the kept triangles
-// in ascending id), as the restatement sums.
+// A block of kMixWarps warps per polyhedron.  A polyhedron is a long chain of
+// tests (the spheres around it, the polyhedra around it one at a time, the
+// triangles near it one at a time), and a charge has few of them: with a warp
+// each, 1,000 rocks filled 8 % of the warp slots and the step took as long as
+// the rock with the most neighbours and triangles.  Here the tests are tasks
+// that the block's warps take in turn (1,000 rocks among 20,000 balls in the
+// turning drum, 32 steps: 1.49 -> 1.37 ms, one state alone 3.58 -> 3.15).  Every test is
+// evaluated as one warp did, and the results are summed in the same order:
+// the polyhedron's own force by one lane in slot order, then the walls
+// (planes in order, then the kept triangles in ascending id), as the
+// restatement sums.
 template <bool kCapture, bool kRot>
-__global__ void __launch_bounds__(32 * kMixWarps, 4)
+__global__ void __launch_bounds__(kMixBlock, 4)
 k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_sorted,
                 StateBuf out, StepCtl* ctl, StepLink link, EnsCapture cap) {
-  __shared__ MixSmem smem[kMixWarps];
-  const int lane = threadIdx.x & 31;
-  MixSmem& sm = smem[threadIdx.x >> 5];
-  const int p = blockIdx.x * kMixWarps + (int)(threadIdx.x >> 5);
-  if (p >= m.npoly) return;
+  __shared__ MixSmem sm;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int p = blockIdx.x;
   const bool rebuilt = *link.rebuilt != 0;
   const StateBuf in = rebuilt ? in_sorted : in_plain;
   const int e = ctl->epoch & 1;
@@ -395,19 +414,33 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
   const uint32_t mlo = L.mlo[p], mhi = L.mhi[p];
   uint32_t st = 0;
 
-  // sphere neighbours: a slot per lane
-  uint32_t touch[2], polys[2];
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
+  // the polyhedra whose bounding spheres overlap this one's (two warps, a
+  // slot per lane)
+  if (threadIdx.x < 2) sm.touch[threadIdx.x] = 0u;
+  if (wid < 2) {
+    const uint32_t k = (uint32_t)threadIdx.x;
+    bool pair = false;
+    if (k < cnt) {
+      const float4 pb4 = in.pos[L.idx[(size_t)k * P + p]];
+      if (pb4.w < 0.0f) {
+        const float3 rel = xyz(pb4) - xa;
+        const float sr = rb - pb4.w;
+        pair = dot3(rel, rel) < sr * sr;
+      }
+    }
+    const uint32_t bal = __ballot_sync(0xffffffffu, pair);
+    if (lane == 0) sm.polys[wid] = bal;
+  }
+
+  // a sphere neighbour per lane, slots 32 half + lane
+  auto spheres = [&](int half) {
     const uint32_t k = (uint32_t)lane + 32u * (uint32_t)half;
-    bool is_poly = false, touched = false;
+    bool touched = false;
     if (k < cnt) {
       const size_t sk = (size_t)k * P + p;
       const uint32_t j = L.idx[sk];
       const float4 pb4 = in.pos[j];
-      if (pb4.w < 0.0f) {
-        is_poly = true;
-      } else {
+      if (!(pb4.w < 0.0f)) {
         // the pair is evaluated here only: the sphere's step reads the force
         // and torque on it from sf / st
         const float3 rel = xyz(pb4) - xa;
@@ -436,69 +469,59 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
         m.st[sk] = sto;
       }
     }
-    touch[half] = __ballot_sync(0xffffffffu, touched);
-    polys[half] = __ballot_sync(0xffffffffu, is_poly);
-  }
+    const uint32_t bal = __ballot_sync(0xffffffffu, touched);
+    if (lane == 0 && bal) atomicOr(&sm.touch[half], bal);
+  };
 
-  // polyhedron neighbours: the warp on one pair at a time
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {
-    uint32_t pm = polys[half];
-    while (pm) {
-      const int bit = __ffs(pm) - 1;
-      pm &= pm - 1u;
-      const uint32_t k = (uint32_t)bit + 32u * (uint32_t)half;
-      const size_t sk = (size_t)k * P + p;
-      const uint32_t j = L.idx[sk];
-      const float4 pb4 = in.pos[j], vb4 = in.vel[j], wb4 = in.angv[j];
-      const int q = __float_as_int(wb4.w);
-      const int sq = m.shape_of[q];
-      const bool selfA = p < q;
-      const float3 xA = selfA ? xa : xyz(pb4), xB = selfA ? xyz(pb4) : xa;
-      const float rA = selfA ? rb : -pb4.w, rB = selfA ? -pb4.w : rb;
-      const float3 rel = xB - xA;
-      const float sr = rA + rB;
-      if (!(dot3(rel, rel) < sr * sr)) continue;
-      HullRef Bq;
-      Bq.V = m.gv + (size_t)q * kMixMaxV;
-      Bq.F = m.gf + (size_t)q * kMixMaxF;
-      Bq.E = m.edges + (size_t)sq * kMixMaxE;
-      Bq.nv = m.shapes[sq].nv;
-      Bq.nf = m.shapes[sq].nf;
-      Bq.ne = m.shapes[sq].ne;
-      const HullRef& HA = selfA ? A : Bq;
-      const HullRef& HB = selfA ? Bq : A;
-      const double3 d = dsub(d3(xB), d3(xA));
-      const int code = L.sep[sk];
-      if (code >= 0 && axis_separates(code, d, HA, HB)) continue;
-      SatPick pick;
-      int scode;
-      if (!hull_hull_warp(lane, d, HA, HB, pick, scode)) {
-        if (lane == 0 && scode != code) L.sep[sk] = scode;
-        continue;
-      }
-      MixHit h;
-      if (!hull_hull_finish(pick, d, HA.V, HA.F, HA.E, HA.nv, HB.V, HB.F, HB.E, HB.nv, HB.ne, h))
-        continue;
-      if (lane == 0) {
-        float3 xi = f3(0.0f, 0.0f, 0.0f);
-        if ((((half ? mhi : mlo) >> bit) & 1u) != 0u) xi = f3(L.hx[sk], L.hy[sk], L.hz[sk]);
-        const float mq = m.shapes[sq].mass;
-        float3 F, TA, TB;
-        if (selfA) mix_pair_law(S, h, mass, va, wa, mq, xyz(vb4), xyz(wb4), dt, xi, F, TA, TB);
-        else mix_pair_law(S, h, mq, xyz(vb4), xyz(wb4), mass, va, wa, dt, xi, F, TA, TB);
-        L.hx[sk] = xi.x;
-        L.hy[sk] = xi.y;
-        L.hz[sk] = xi.z;
-        sm.f[k] = selfA ? make_float4(F.x, F.y, F.z, 0.0f) : make_float4(-F.x, -F.y, -F.z, 0.0f);
-        sm.t[k] = selfA ? make_float4(TA.x, TA.y, TA.z, 0.0f) : make_float4(TB.x, TB.y, TB.z, 0.0f);
-      }
-      touch[half] |= 1u << bit;
+  // the polyhedron in slot k, by the warp
+  auto poly_pair = [&](uint32_t k) {
+    const uint32_t bit = k & 31u, half = k >> 5;
+    const size_t sk = (size_t)k * P + p;
+    const uint32_t j = L.idx[sk];
+    const float4 pb4 = in.pos[j], vb4 = in.vel[j], wb4 = in.angv[j];
+    const int q = __float_as_int(wb4.w);
+    const int sq = m.shape_of[q];
+    const bool selfA = p < q;
+    const float3 xA = selfA ? xa : xyz(pb4), xB = selfA ? xyz(pb4) : xa;
+    HullRef Bq;
+    Bq.V = m.gv + (size_t)q * kMixMaxV;
+    Bq.F = m.gf + (size_t)q * kMixMaxF;
+    Bq.E = m.edges + (size_t)sq * kMixMaxE;
+    Bq.nv = m.shapes[sq].nv;
+    Bq.nf = m.shapes[sq].nf;
+    Bq.ne = m.shapes[sq].ne;
+    const HullRef& HA = selfA ? A : Bq;
+    const HullRef& HB = selfA ? Bq : A;
+    const double3 d = dsub(d3(xB), d3(xA));
+    const int code = L.sep[sk];
+    if (code >= 0 && axis_separates(code, d, HA, HB)) return;
+    SatPick pick;
+    int scode;
+    if (!hull_hull_warp(lane, d, HA, HB, pick, scode)) {
+      if (lane == 0 && scode != code) L.sep[sk] = scode;
+      return;
     }
-  }
+    MixHit h;
+    if (!hull_hull_finish(pick, d, HA.V, HA.F, HA.E, HA.nv, HB.V, HB.F, HB.E, HB.nv, HB.ne, h))
+      return;
+    if (lane == 0) {
+      float3 xi = f3(0.0f, 0.0f, 0.0f);
+      if ((((half ? mhi : mlo) >> bit) & 1u) != 0u) xi = f3(L.hx[sk], L.hy[sk], L.hz[sk]);
+      const float mq = m.shapes[sq].mass;
+      float3 F, TA, TB;
+      if (selfA) mix_pair_law(S, h, mass, va, wa, mq, xyz(vb4), xyz(wb4), dt, xi, F, TA, TB);
+      else mix_pair_law(S, h, mq, xyz(vb4), xyz(wb4), mass, va, wa, dt, xi, F, TA, TB);
+      L.hx[sk] = xi.x;
+      L.hy[sk] = xi.y;
+      L.hz[sk] = xi.z;
+      sm.f[k] = selfA ? make_float4(F.x, F.y, F.z, 0.0f) : make_float4(-F.x, -F.y, -F.z, 0.0f);
+      sm.t[k] = selfA ? make_float4(TA.x, TA.y, TA.z, 0.0f) : make_float4(TB.x, TB.y, TB.z, 0.0f);
+      atomicOr(&sm.touch[half], 1u << bit);
+    }
+  };
 
-  // triangles: a candidate per lane, in the drum's frame when it turns
-  int nhit = 0;
+  // candidate triangles, in the drum's frame when it turns
+  int nhit = 0;             // touching triangles (the block's)
   bool rot = false;
   float rc = 1.0f, rsn = 0.0f;
   if constexpr (kRot) {
@@ -509,149 +532,228 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
       rsn = cs.y;
     }
   }
+  uint32_t o0 = 0, o1 = 0;
+  const float3 pd = rot ? S.rot_o + rot_about(S.rot_a, rc, -rsn, xa - S.rot_o) : xa;
   if (g.tri_off) {
-    const float3 pd = rot ? S.rot_o + rot_about(S.rot_a, rc, -rsn, xa - S.rot_o) : xa;
     const int3 c = ens_cell(S, pd);
     if (ens_in(S, c)) {
       const uint32_t hcell = ens_key(S, c);
-      const uint32_t o0 = __ldg(g.tri_off + hcell), o1 = __ldg(g.tri_off + hcell + 1);
-      if (o1 > o0) {
-        HullRef D = A;
-        if (rot) {
-          const double3 ax = d3(S.rot_a);
-          const double cc = (double)rc, ss = -(double)rsn;
-          for (int it = lane; it < A.nv + A.nf; it += 32) {
-            if (it < A.nv) {
-              const double3 v = rot_about_d(ax, cc, ss, dxyz(A.V[it]));
-              sm.v[it] = make_double4(v.x, v.y, v.z, 0.0);
-            } else {
-              const double4 P4 = A.F[it - A.nv];
-              const double3 n = rot_about_d(ax, cc, ss, dxyz(P4));
-              sm.fn[it - A.nv] = make_double4(n.x, n.y, n.z, P4.w);
-            }
-          }
-          __syncwarp();
-          D.V = sm.v;
-          D.F = sm.fn;
-        }
-        // candidates near the polyhedron (a lane each), then the test of
-        // each, in ascending order, by the whole warp
-        const float lim = rb * 1.001f + 1e-3f;
-        for (uint32_t q0 = o0; q0 < o1; q0 += 32) {
-          const uint32_t qq = q0 + (uint32_t)lane;
-          bool near = false;
-          int id = -1;
-          if (qq < o1) {
-            id = (int)__ldg(g.tri_ids + qq);
-            const EnsWallDev& W = g.walls[id];
-            int region, feat;
-            const float3 cp = closest_on_triangle(pd, W.a, W.b, W.c, region, feat);
-            const float3 dd = pd - cp;
-            near = dot3(dd, dd) < lim * lim;
-          }
-          uint32_t nb = __ballot_sync(0xffffffffu, near);
-          while (nb) {
-            const int src = __ffs(nb) - 1;
-            nb &= nb - 1u;
-            const int tid = __shfl_sync(0xffffffffu, id, src);
-            const EnsWallDev& W = g.walls[tid];
-            const double3 o = d3(pd);
-            double3 T[3];
-            T[0] = dsub(d3(W.a), o);
-            T[1] = dsub(d3(W.b), o);
-            T[2] = dsub(d3(W.c), o);
-            MixHit h;
-            double3 nd;
-            int kind;
-            if (!hull_tri_warp(lane, D, T, W.n64, h, nd, kind)) continue;
-            if (lane == 0 && nhit < kMixHits) {
-              sm.hit[nhit] = h;
-              sm.nd[nhit] = nd;
-              sm.hid[nhit] = tid;
-              sm.hkind[nhit] = kind;
-            }
-            ++nhit;
-          }
-        }
-        if (nhit > kMixHits) {
-          st |= kStatusListOverflow;
-          nhit = kMixHits;
-        }
-        __syncwarp();
-      }
+      o0 = __ldg(g.tri_off + hcell);
+      o1 = __ldg(g.tri_off + hcell + 1);
     }
   }
-
-  if (lane == 0) {
-    float3 f = f3(0.0f, 0.0f, 0.0f), t = f3(0.0f, 0.0f, 0.0f);
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint32_t tm = touch[half];
-      while (tm) {
-        const int k = __ffs(tm) - 1 + 32 * half;
-        tm &= tm - 1u;
-        f = f + xyz(sm.f[k]);
-        t = t + xyz(sm.t[k]);
+  HullRef D = A;
+  if (o1 > o0 && rot) {
+    const double3 ax = d3(S.rot_a);
+    const double cc = (double)rc, ss = -(double)rsn;
+    for (int it = (int)threadIdx.x; it < A.nv + A.nf; it += kMixBlock) {
+      if (it < A.nv) {
+        const double3 v = rot_about_d(ax, cc, ss, dxyz(A.V[it]));
+        sm.v[it] = make_double4(v.x, v.y, v.z, 0.0);
+      } else {
+        const double4 P4 = A.F[it - A.nv];
+        const double3 n = rot_about_d(ax, cc, ss, dxyz(P4));
+        sm.fn[it - A.nv] = make_double4(n.x, n.y, n.z, P4.w);
       }
     }
-    if (touch[0] != mlo) L.mlo[p] = touch[0];
-    if (touch[1] != mhi) L.mhi[p] = touch[1];
+    D.V = sm.v;
+    D.F = sm.fn;
+  }
+  // Windows of kMixBlock candidate triangles; the first window's tasks are
+  // also the spheres and the polyhedra.
+  const float lim = rb * 1.001f + 1e-3f;
+  bool first = true;
+  for (uint32_t q0 = o0; first || q0 < o1; q0 += kMixBlock, first = false) {
+    const uint32_t qq = q0 + threadIdx.x;
+    bool near = false;
+    int id = -1;
+    if (qq < o1) {
+      const float4 bs = __ldg(g.tri_b + qq);
+      const float3 dc = pd - xyz(bs);
+      const float reach = bs.w + lim;
+      if (!(dot3(dc, dc) > reach * reach)) {
+        id = (int)__ldg(g.tri_ids + qq);
+        const EnsWallDev& W = g.walls[id];
+        int region, feat;
+        const float3 cp = closest_on_triangle(pd, W.a, W.b, W.c, region, feat);
+        const float3 dd = pd - cp;
+        near = dot3(dd, dd) < lim * lim;
+      }
+    }
+    const uint32_t nb = __ballot_sync(0xffffffffu, near);
+    if (lane == 0) sm.nearby[wid] = nb;
+    if (threadIdx.x == 0) sm.task = 0;
+    __syncthreads();
+    int at = 0, nnear = 0;
+#pragma unroll
+    for (int w = 0; w < kMixWarps; ++w) {
+      if (w < wid) at += __popc(sm.nearby[w]);
+      nnear += __popc(sm.nearby[w]);
+    }
+    if (near) sm.id[at + __popc(nb & ((1u << lane) - 1u))] = id;
+    __syncthreads();
+    const uint32_t pl = first ? sm.polys[0] : 0u, ph = first ? sm.polys[1] : 0u;
+    const int nsph = first ? (cnt > 32u ? 2 : 1) : 0;
+    const int npair = __popc(pl) + __popc(ph);
+    const int tasks = npair + nsph + nnear;
+    for (;;) {
+      int t = 0;
+      if (lane == 0) t = atomicAdd(&sm.task, 1);
+      t = __shfl_sync(0xffffffffu, t, 0);
+      if (t >= tasks) break;
+      if (t < nsph) {
+        spheres(t);
+      } else if (t < nsph + npair) {
+        int r = t - nsph;
+        uint32_t word = pl, base = 0u;
+        if (r >= __popc(pl)) {
+          r -= __popc(pl);
+          word = ph;
+          base = 32u;
+        }
+        for (; r > 0; --r) word &= word - 1u;
+        poly_pair(base + (uint32_t)__ffs(word) - 1u);
+      } else {
+        const int r = t - nsph - npair;
+        const EnsWallDev& W = g.walls[sm.id[r]];
+        const double3 o = d3(pd);
+        double3 T[3];
+        T[0] = dsub(d3(W.a), o);
+        T[1] = dsub(d3(W.b), o);
+        T[2] = dsub(d3(W.c), o);
+        MixHit h;
+        double3 nd;
+        int kind = -1;
+        const bool hit = hull_tri_warp(lane, D, T, W.n64, h, nd, kind);
+        if (lane == 0) {
+          sm.kind[r] = hit ? kind : -1;
+          if (hit) {
+            sm.hit[r] = h;
+            sm.nd[r] = nd;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    // the window's touching triangles behind the earlier ones
+    for (int r0 = 0; r0 < nnear; r0 += 32) {
+      const int r = r0 + lane;
+      const bool hit = r < nnear && sm.kind[r] >= 0;
+      const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+      const int to = nhit + __popc(bal & ((1u << lane) - 1u));
+      if (wid == 0 && hit && to < kMixHits) {
+        sm.khit[to] = sm.hit[r];
+        sm.knd[to] = sm.nd[r];
+        sm.kid[to] = sm.id[r];
+        sm.kkind[to] = sm.kind[r];
+      }
+      nhit += __popc(bal);
+    }
+    __syncthreads();
+  }
+  if (wid != 0) return;     // one warp sums and integrates
+  if (nhit > kMixHits) {
+    st |= kStatusListOverflow;
+    nhit = kMixHits;
+  }
 
-    // walls: the old history slots (by wall id), new ones written in
-    // processing order over them
-    float4* wh = m.wh + (size_t)p * kMixWallSlots;
-    const int nw_o = m.wn[p];
-    float4* oh = sm.oh;
-    for (int qs = 0; qs < nw_o; ++qs) oh[qs] = wh[qs];
-    int nw = 0;
-    auto wall = [&](int id, const MixHit& h, bool moving) {
+  float3 f = f3(0.0f, 0.0f, 0.0f), t = f3(0.0f, 0.0f, 0.0f);
+  // the contacts in slot order (every lane the same sum)
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    uint32_t tm = sm.touch[half];
+    while (tm) {
+      const int k = __ffs(tm) - 1 + 32 * half;
+      tm &= tm - 1u;
+      f = f + xyz(sm.f[k]);
+      t = t + xyz(sm.t[k]);
+    }
+  }
+  if (lane == 0) {
+    if (sm.touch[0] != mlo) L.mlo[p] = sm.touch[0];
+    if (sm.touch[1] != mhi) L.mhi[p] = sm.touch[1];
+  }
+
+  // walls, a contact per lane: the old history slots (by wall id) read
+  // first, the new ones written in processing order over them, the forces
+  // added in processing order
+  float4* wh = m.wh + (size_t)p * kMixWallSlots;
+  const int nw_o = m.wn[p];
+  if (lane < nw_o) sm.oh[lane] = wh[lane];
+  __syncwarp();
+  int nw = 0;
+  auto walls = [&](bool hit, int id, const MixHit& h, bool moving) {
+    const uint32_t bal = __ballot_sync(0xffffffffu, hit);
+    if (hit) {
+      const int slot = nw + __popc(bal & ((1u << lane) - 1u));
       float3 xi = f3(0.0f, 0.0f, 0.0f);
       for (int qs = 0; qs < nw_o; ++qs)
-        if (__float_as_int(oh[qs].w) == id) xi = f3(oh[qs].x, oh[qs].y, oh[qs].z);
+        if (__float_as_int(sm.oh[qs].w) == id) xi = xyz(sm.oh[qs]);
       const float3 vw = moving ? cross3(S.rot_a, (xa + h.ca) - S.rot_o) * S.rot_w
                                : f3(0.0f, 0.0f, 0.0f);
       float3 F, T;
       mix_wall_law(S, h, mass, va, wa, vw, dt, xi, F, T);
-      f = f + F;
-      t = t + T;
-      if (nw < kMixWallSlots) {
-        wh[nw] = make_float4(xi.x, xi.y, xi.z, __int_as_float(id));
-        ++nw;
-      } else {
-        st |= kStatusListOverflow;
-      }
-    };
-    for (int w = S.wall0; w < S.wall0 + S.nwall; ++w) {
+      sm.wf[lane] = make_float4(F.x, F.y, F.z, 0.0f);
+      sm.wt[lane] = make_float4(T.x, T.y, T.z, 0.0f);
+      if (slot < kMixWallSlots) wh[slot] = make_float4(xi.x, xi.y, xi.z, __int_as_float(id));
+      else st |= kStatusListOverflow;
+    }
+    __syncwarp();
+    for (uint32_t w = bal; w; w &= w - 1u) {
+      f = f + xyz(sm.wf[__ffs(w) - 1]);
+      t = t + xyz(sm.wt[__ffs(w) - 1]);
+    }
+    __syncwarp();
+    nw = min(nw + __popc(bal), kMixWallSlots);
+  };
+  for (int w0 = 0; w0 < S.nwall; w0 += 32) {
+    const int w = S.wall0 + w0 + lane;
+    MixHit h;
+    bool hit = false, moving = false;
+    if (w0 + lane < S.nwall) {
       const EnsWallDev& W = g.walls[w];
-      MixHit h;
-      if (W.kind == kWallPlane && hull_plane(W.a, W.r, xa, A.V, A.nv, h))
-        wall(w, h, rot && W.turning);
+      hit = W.kind == kWallPlane && hull_plane(W.a, W.r, xa, A.V, A.nv, h);
+      moving = rot && W.turning;
     }
-    // contacts with a triangle's face all count, those of one plane once
-    // (the deepest); without one, only the deepest other contact does (a
-    // polyhedron over the shared edge of two triangles of a flat or concave
-    // region touches it once)
-    bool anyface = false;
-    int best = -1;
-    for (int a = 0; a < nhit; ++a) {
-      if (sm.hkind[a] == 0) anyface = true;
-      else if (best < 0 || sm.hit[a].delta > sm.hit[best].delta) best = a;
-    }
-    for (int a = 0; a < nhit; ++a) {
-      bool keep = anyface ? sm.hkind[a] == 0 : a == best;
-      for (int c2 = 0; c2 < nhit && keep && anyface; ++c2) {
-        if (c2 == a || sm.hkind[c2] != 0 || !(ddot(sm.nd[a], sm.nd[c2]) > kMixCoplanar)) continue;
-        const float da = sm.hit[a].delta, dc = sm.hit[c2].delta;
-        if (dc > da || (dc == da && sm.hid[c2] < sm.hid[a])) keep = false;
+    walls(hit, w, h, moving);
+  }
+  // contacts with a triangle's face all count, those of one plane once
+  // (the deepest); without one, only the deepest other contact does (a
+  // polyhedron over the shared edge of two triangles of a flat or concave
+  // region touches it once)
+  if (nhit > 0) {
+    const bool have = lane < nhit;
+    const int kind = have ? sm.kkind[lane] : -1;
+    const float da = have ? sm.khit[lane].delta : 0.0f;
+    const bool anyface = __any_sync(0xffffffffu, kind == 0);
+    // the first of the deepest contacts that are not on a triangle's face
+    const bool edge = have && kind != 0;
+    const float dmax = __uint_as_float(
+        __reduce_max_sync(0xffffffffu, edge ? __float_as_uint(da) : 0u));   // depths are positive
+    const uint32_t deepest = __ballot_sync(0xffffffffu, edge && da == dmax);
+    bool keep = have && (anyface ? kind == 0 : lane == __ffs(deepest) - 1);
+    if (keep && anyface) {
+      for (int c2 = 0; c2 < nhit && keep; ++c2) {
+        if (c2 == lane || sm.kkind[c2] != 0 || !(ddot(sm.knd[lane], sm.knd[c2]) > kMixCoplanar))
+          continue;
+        const float dc = sm.khit[c2].delta;
+        if (dc > da || (dc == da && sm.kid[c2] < sm.kid[lane])) keep = false;
       }
-      if (!keep) continue;
-      MixHit h = sm.hit[a];
+    }
+    MixHit h;
+    int id = -1;
+    if (keep) {
+      h = sm.khit[lane];
+      id = sm.kid[lane];
       if (rot) {
         h.n = rot_about(S.rot_a, rc, rsn, h.n);
         h.ca = rot_about(S.rot_a, rc, rsn, h.ca);
       }
-      wall(sm.hid[a], h, rot);
     }
+    walls(keep, id, h, rot);
+  }
+
+  if (lane == 0) {
     m.wn[p] = nw;
 
     // symplectic Euler: translation; rotation by Euler's equations in the
@@ -739,14 +841,14 @@ void mix_launch_poly_step(const EnsGeom& g, const EnsBufs& b, const MixBufs& m, 
                           StepCtl* ctl, StepLink link, const EnsCapture* cap, cudaStream_t st) {
   if (m.npoly <= 0) return;
   const EnsCapture c = cap ? *cap : EnsCapture{nullptr, nullptr};
-  const int gs = (m.npoly + kMixWarps - 1) / kMixWarps;
+  const int gs = m.npoly;
 #define MIX_ARGS g, b, m, b.S[cur], b.S[2], b.S[cur ^ 1], ctl, link, c
   if (g.any_rot) {
-    if (cap) k_mix_poly_step<true, true><<<gs, 32 * kMixWarps, 0, st>>>(MIX_ARGS);
-    else k_mix_poly_step<false, true><<<gs, 32 * kMixWarps, 0, st>>>(MIX_ARGS);
+    if (cap) k_mix_poly_step<true, true><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
+    else k_mix_poly_step<false, true><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
   } else {
-    if (cap) k_mix_poly_step<true, false><<<gs, 32 * kMixWarps, 0, st>>>(MIX_ARGS);
-    else k_mix_poly_step<false, false><<<gs, 32 * kMixWarps, 0, st>>>(MIX_ARGS);
+    if (cap) k_mix_poly_step<true, false><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
+    else k_mix_poly_step<false, false><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
   }
 #undef MIX_ARGS
 }
