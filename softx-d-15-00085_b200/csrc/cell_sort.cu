@@ -40,8 +40,9 @@ __device__ __forceinline__ uint32_t tiles_before(const uint32_t* tile, uint32_t 
 // A block per tile of cells, and a last one for the particles without a
 // cell: their blocks' counts become positions.
 __global__ void __launch_bounds__(kScanThreads)
-k_cell_scan(CellSort c, int nblocks, const int* gate) {
+k_cell_scan(CellSort c, int nblocks, int* clear, const int* gate) {
   if (gate != nullptr && *gate == 0) return;
+  if (clear && blockIdx.x == 0 && threadIdx.x == 0) *clear = 0;
   __shared__ uint32_t sh[kScanThreads / 32];
   const uint32_t tiles = cell_tiles(c.ncell);
   const uint32_t t = blockIdx.x;
@@ -99,9 +100,10 @@ k_cell_place(CellSort c, int n, int* epoch, const int* gate) {
 
 }  // namespace
 
-void cell_scan_place(const CellSort& c, int n, int* epoch, const int* gate, cudaStream_t stream) {
+void cell_scan_place(const CellSort& c, int n, int* epoch, int* clear, const int* gate,
+                     cudaStream_t stream) {
   const int nb = sort_blocks(n);
-  k_cell_scan<<<cell_tiles(c.ncell) + 1u, kScanThreads, 0, stream>>>(c, nb, gate);
+  k_cell_scan<<<cell_tiles(c.ncell) + 1u, kScanThreads, 0, stream>>>(c, nb, clear, gate);
   k_cell_place<<<nb, kSortThreads, 0, stream>>>(c, n, epoch, gate);
 }
 

@@ -108,10 +108,11 @@ __device__ __forceinline__ int cell_dest(const CellSort& c, int i, bool valid) {
 }
 
 // The scan and place passes over n particles; *epoch (may be null) is
-// incremented.  `gate` (may be null): when non-null and *gate == 0 every
-// kernel returns at once, so the launch sequence can stay fixed while the
-// work is skipped.
-void cell_scan_place(const CellSort& c, int n, int* epoch, const int* gate, cudaStream_t stream);
+// incremented and *clear (may be null) set to 0.  `gate` (may be null): when
+// non-null and *gate == 0 every kernel returns at once, so the launch
+// sequence can stay fixed while the work is skipped.
+void cell_scan_place(const CellSort& c, int n, int* epoch, int* clear, const int* gate,
+                     cudaStream_t stream);
 constexpr int kCellSortKernels = 2;
 
 }  // namespace blaze

@@ -145,8 +145,10 @@ __global__ void k_gate_graph(StepCtl* ctl, cudaGraphConditionalHandle h0, int* r
 // out of range) and raises kStatusOutOfGrid.
 __global__ void __launch_bounds__(kSortThreads)
 k_hash(const SimParams* __restrict__ P, const float4* __restrict__ pos, OrderBuf ob, int n_max,
-       CellSort cs, StepCtl* ctl, const int* gate) {
-  if (gate && *gate == 0) return;
+       CellSort cs, StepCtl* ctl, const int* gate, int* latch) {
+  const int req = gate ? *gate : 1;
+  if (latch && blockIdx.x == 0 && threadIdx.x == 0) *latch = req;
+  if (req == 0) return;
   const int i = blockIdx.x * kSortThreads + threadIdx.x;
   const bool valid = i < n_max;
   uint32_t key = 0;
@@ -953,8 +955,8 @@ void launch_gate_graph(StepCtl* ctl, cudaGraphConditionalHandle h0, int* rb, int
 }
 
 void launch_hash(const SimParams* dp, const StateBuf& s, const OrderBuf& ob, int n_max,
-                 const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_hash<<<sort_blocks(n_max), kSortThreads, 0, st>>>(dp, s.pos, ob, n_max, cs, ctl, gate);
+                 const CellSort& cs, StepCtl* ctl, const int* gate, int* latch, cudaStream_t st) {
+  k_hash<<<sort_blocks(n_max), kSortThreads, 0, st>>>(dp, s.pos, ob, n_max, cs, ctl, gate, latch);
 }
 
 void launch_reorder(const StateBuf& src, const StateBuf& dst, const OrderBuf& ob, int n_max,

@@ -146,8 +146,9 @@ void launch_gate_body(StepCtl* ctl, cudaGraphConditionalHandle h0, cudaStream_t 
 // graph: its decision also sets the IF node `h` of the step's re-sort.
 void launch_gate_if(StepCtl* ctl, cudaGraphConditionalHandle h, float skin, float look,
                     int block_start, float vwall, cudaStream_t st);
+// (*latch, when given, takes the gate's value for the kernels after it)
 void launch_hash(const SimParams* dp, const StateBuf& s, const OrderBuf& ob, int n_max,
-                 const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st);
+                 const CellSort& cs, StepCtl* ctl, const int* gate, int* latch, cudaStream_t st);
 // (flat_n, when given, is reset for the contact-list kernel's flat list)
 void launch_reorder(const StateBuf& src, const StateBuf& dst, const OrderBuf& ob, int n_max,
                     const CellSort& cs, bool has_lift, int* flat_n, StepCtl* ctl, const int* gate,

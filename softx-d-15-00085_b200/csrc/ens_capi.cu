@@ -445,7 +445,7 @@ int enqueue_rebuild(blaze_ens* e, const int* gate, cudaStream_t st) {
   const int n = e->n;
   const EnsGeom g = geom(e);
   ens_launch_hash(g, e->b, e->cur, n, e->cs, e->ctl, gate, st);
-  cell_scan_place(e->cs, n, &e->ctl->epoch, gate, st);
+  cell_scan_place(e->cs, n, &e->ctl->epoch, nullptr, gate, st);
   ens_launch_reorder(e->b, e->cur, n, e->cs, e->ctl, gate, st);
   ens_launch_nlist(g, e->b, n, e->cs, e->ctl, gate, st);
   if (e->npoly > 0) {

@@ -188,8 +188,8 @@ extern "C" int blaze_contact_list_static(const float* pos4, int n, const Simulat
   CKS(cudaMemsetAsync(ob.pid[0], 0, sizeof(int) * n, st));  // every particle live
   CKS(cudaMemsetAsync(cs.cnt, 0, sizeof(uint32_t) * (size_t)cell_tiles(cs.ncell) * kTileCells, st));
   CKS(cudaMemsetAsync(cs.tile, 0, sizeof(uint32_t) * (cell_tiles(cs.ncell) + 1), st));
-  launch_hash(dp, src, ob, n, cs, ctl, nullptr, st);
-  cell_scan_place(cs, n, nullptr, nullptr, st);
+  launch_hash(dp, src, ob, n, cs, ctl, nullptr, nullptr, st);
+  cell_scan_place(cs, n, nullptr, nullptr, nullptr, st);
   launch_reorder(src, dst, ob, n, cs, false, nullptr, ctl, nullptr, st);
   NbrList nl;
   nl.idx = list;
