@@ -95,6 +95,7 @@ struct blaze_sim {
   // objects, world objects, FP64 on the device; per-particle values of the
   // step and per-block partial sums when the step computes them
   double* d_tally = nullptr;
+  unsigned int* d_done = nullptr;      // blocks of the running step that are done (StepTail)
   double* d_eb = nullptr;
   double* d_epart = nullptr;
   float fc = 0.0f;
@@ -595,12 +596,17 @@ cudaEvent_t prof_event(blaze_sim* s, int phase) {
 // The kernels of one step after the (conditional) re-sort, reading S[cur]
 // or the sorted copy S[2] as `link` says and writing S[cur ^ 1]; returns the
 // number of launches.
-int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st) {
+// first / last: of the steps launched together (a graph's); with energy
+// tallies the step before moves a step's volume objects (StepTail::next).
+int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st, bool first = true,
+                         bool last = true) {
   const ForceCapture* cap = s->opt.capture_forces ? &s->cap : nullptr;
   int k = 1;
-  if (s->dobj_rot || s->dobj_tr >= 0) {
-    launch_move_dobj(s->dp, s->dobj_rot ? 1 : 0, s->rot_ax, s->rot_ay, s->rot_c, s->rot_s,
-                     s->dobj_tr, s->n_d, st);
+  const bool moves = (s->dobj_rot || s->dobj_tr >= 0) && s->n_d > 0;
+  const DobjMove mv{s->dobj_rot ? 1 : 0, s->dobj_tr, s->rot_ax, s->rot_ay, s->rot_c, s->rot_s};
+  const bool energy = s->hp.energy_calc && s->d_epart;   // allocated when EnergyCalc
+  if (moves && (first || s->poly || !energy)) {
+    launch_move_dobj(s->dp, mv, s->n_d, st);
     ++k;
   }
   if (s->wobj_rot) {
@@ -608,7 +614,7 @@ int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st) {
                        s->wrot_c, s->wrot_s, st);
     ++k;
   }
-  double* eb = s->hp.energy_calc ? s->d_eb : nullptr;   // allocated when EnergyCalc
+  double* eb = energy ? s->d_eb : nullptr;
   if (s->poly) {
     launch_poly_geom(s->d_shapes, s->geom, s->S[s->cur], s->S[2], s->ob, s->n_max,
                      s->si.Rotation ? 1 : 0, s->ctl, link.rebuilt, st);
@@ -619,11 +625,12 @@ int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st) {
                      st);
     k += 1 + np;
   } else {
+    const StepTail tail{s->d_done, s->d_epart, s->d_tally, s->dp, mv, moves && !last ? 1 : 0};
     launch_step(s->dp, s->d_ops, WallGrid{s->d_wall_off, s->d_wall_idx}, s->S[s->cur], s->S[2],
-                s->S[s->cur ^ 1], s->ob, s->n_max, s->nl, s->ctl, link, s->spin_free, cap, eb,
-                s->opt.fast_law != 0, st);
+                s->S[s->cur ^ 1], s->ob, s->n_max, s->nl, s->ctl, link, s->spin_free, cap, energy,
+                tail, s->opt.fast_law != 0, st);
   }
-  if (eb) {
+  if (s->poly && eb) {
     launch_energy_reduce(eb, s->n_max, s->ctl, s->d_epart, s->d_tally, st);
     k += 2;
   }
@@ -826,7 +833,9 @@ int build_graph(blaze_sim* s, int c, int steps, cudaGraphExec_t* out_exec) {
                                    cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < steps; ++k) {
     enqueue_reference_rebuild(s, s->stream);
-    s->step_launches = enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream);
+    const int ks = enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream, k == 0,
+                                        k + 1 == steps);
+    if (k == 0) s->step_launches = ks;
     s->cur ^= 1;
   }
   cudaGraph_t out = nullptr;
@@ -865,7 +874,7 @@ int capture_block_body(blaze_sim* s, cudaGraph_t body, cudaStream_t bs, cudaStre
     if (k < n_if) rc = add_rebuild_if(s, bs, bs2, h[k], k);
     const StepLink link = k + 1 < n_if ? StepLink{s->d_rb + k, h[k + 1], 1, 0}
                                         : StepLink{s->d_rb + k, 0, 0, (int)(k + 1 == kGraphSteps)};
-    s->step_launches = enqueue_step_kernels(s, link, bs);
+    s->step_launches = enqueue_step_kernels(s, link, bs, k == 0, k + 1 == kGraphSteps);
     s->cur ^= 1;
   }
   cudaGraph_t tmp = nullptr;
@@ -1073,7 +1082,7 @@ void free_sim(blaze_sim* s) {
   for (int b = 0; b < 3; ++b) { f(s->S[b].pos); f(s->S[b].vel); f(s->S[b].angv); }
   for (int b = 0; b < 2; ++b) { f(s->ob.pid[b]); f(s->ob.lift[b]); }
   f(s->cs.key); f(s->cs.slot); f(s->cs.member); f(s->cs.cnt); f(s->cs.start); f(s->cs.tile);
-  f(s->cs.spec); f(s->nl.idx); f(s->nl.cnt);
+  f(s->cs.spec); f(s->d_done); f(s->nl.idx); f(s->nl.cnt);
   f(s->ctl); f(s->d_rb); f(s->d_chk); f(s->dp); f(s->d_ops); f(s->d_wall_off); f(s->d_wall_idx);
   f(s->d_tally); f(s->d_eb); f(s->d_epart);
   f(s->cap.f_pp); f(s->cap.t_pp); f(s->cap.f_w); f(s->cap.t_w); f(s->cap.f_l); f(s->cap.t_l);
@@ -1240,10 +1249,12 @@ int create_impl(blaze_sim** out, const WOBJ* w, int n_w, const POBJ* p, int n_p,
   CKF(dalloc(&s->ctl, 1));
   CKF(dalloc(&s->d_rb, kGraphSteps));
   CKF(cudaMemset(s->d_rb, 0, sizeof(int) * kGraphSteps));
+  CKF(dalloc(&s->d_done, 1));
+  CKF(cudaMemset(s->d_done, 0, sizeof(unsigned int)));
   CKF(dalloc(&s->d_tally, 3));
   CKF(cudaMemset(s->d_tally, 0, sizeof(double) * 3));
   if (si->EnergyCalc) {
-    CKF(dalloc(&s->d_eb, (size_t)3 * n));
+    if (si->particle_type == 1) CKF(dalloc(&s->d_eb, (size_t)3 * n));
     CKF(dalloc(&s->d_epart, (size_t)3 * ((n + kEnergyBlock - 1) / kEnergyBlock)));
   }
   CKF(cudaMallocHost((void**)&s->h_ctl, sizeof(StepCtl)));

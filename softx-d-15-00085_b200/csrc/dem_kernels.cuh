@@ -156,29 +156,43 @@ void launch_reorder(const StateBuf& src, const StateBuf& dst, const OrderBuf& ob
 // cell_start: the cell table of the sort (CellSort::start)
 void launch_nlist(const SimParams* dp, const StateBuf& s, int n_max, const uint32_t* cell_start,
                   NbrList nl, StepCtl* ctl, const int* gate, cudaStream_t st);
-// eb: when not null, the step also writes each particle's energy-tally
-// values (particle-particle, volume objects, world objects; FP64) to
-// eb[c * n_max + i].  fast: the contracted particle-particle law (ignored
-// when eb is given: tallies use the reference's arithmetic).
+// One step of the mill driver's moves of volume objects: with `turn`, the
+// drum's turn of the attached ones (c, s: cosine and sine of the step
+// angle, ax, ay: the drum axis); then object `tr` (-1: none) moves by its
+// velocity times dt.
+struct DobjMove {
+  int turn, tr;
+  float ax, ay, c, s;
+};
+// Work of the last block of a step that tallies energy (done: a zeroed
+// counter): tally[c] += the step's values, in a fixed order (part: 3 doubles
+// per block of kEnergyBlock particles), and with `next` the moves that the
+// following step starts with.
+struct StepTail {
+  unsigned int* done;
+  double* part;
+  double* tally;
+  SimParams* params;
+  DobjMove move;
+  int next;
+};
+constexpr int kEnergyBlock = 256;
+// energy: the step tallies energy (with the reference's arithmetic).  fast:
+// the contracted particle-particle law (ignored with `energy`).
 void launch_step(const SimParams* dp, const WallOp* ops, WallGrid wg, const StateBuf& in_plain,
                  const StateBuf& in_sorted, const StateBuf& out, const OrderBuf& ob, int n_max,
                  NbrList nl, StepCtl* ctl, StepLink link, bool spin_free,
-                 const ForceCapture* cap, double* eb, bool fast, cudaStream_t st);
-// tally[c] += sum of eb[c * n_max + i] over the current particles, in a fixed
-// order; part holds 3 doubles per block of kEnergyBlock particles.
-constexpr int kEnergyBlock = 256;
+                 const ForceCapture* cap, bool energy, const StepTail& tail, bool fast,
+                 cudaStream_t st);
+// Polyhedra: tally[c] += sum of eb[c * n_max + i] over the current
+// particles, in the same order; part as in StepTail.
 // Self-check of div3_rn against IEEE division on n random triples:
 // *bad += the components that differ.
 void launch_check_div(long long n, unsigned long long seed, unsigned long long* bad,
                       cudaStream_t st);
 void launch_energy_reduce(const double* eb, int n_max, const StepCtl* ctl, double* part,
                           double* tally, cudaStream_t st);
-// One step of the mill driver's moves of volume objects: with `turn`, the
-// drum's turn of the attached ones (c, s: cosine and sine of the step
-// angle, about: the drum axis); then object `translate` (-1: none) moves by
-// its velocity times dt.
-void launch_move_dobj(SimParams* dp, int turn, float about_x, float about_y, float c, float s,
-                      int translate, int n_dobj, cudaStream_t st);
+void launch_move_dobj(SimParams* dp, const DobjMove& mv, int n_dobj, cudaStream_t st);
 // One step of the turn of the rotating world objects (bit k of rot_mask:
 // world object k) on the wall program.
 void launch_rotate_wobj(WallOp* ops, int n_ops, uint32_t rot_mask, float about_x, float about_y,
