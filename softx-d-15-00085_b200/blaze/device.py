@@ -298,13 +298,13 @@ class Simulation:
         return _check(self.lib.blaze_sync(self.h), "blaze_sync")
 
     def state(self):
-        n = self.n
-        pos = np.zeros((n, 3), np.float32)
-        vel = np.zeros((n, 3), np.float32)
-        avel = np.zeros((n, 3), np.float32)
-        ptype = np.zeros(n, np.uint32)
-        pid = np.zeros(n, np.int32)
-        quat = np.zeros((n, 4), np.float32) if self.poly else None
+        n = self.n   # every entry is written by the library
+        pos = np.empty((n, 3), np.float32)
+        vel = np.empty((n, 3), np.float32)
+        avel = np.empty((n, 3), np.float32)
+        ptype = np.empty(n, np.uint32)
+        pid = np.empty(n, np.int32)
+        quat = np.empty((n, 4), np.float32) if self.poly else None
         st = _check(self.lib.blaze_get_state_ornt(self.h, _ptr(pos, C.c_float),
                                                   _ptr(quat, C.c_float), _ptr(vel, C.c_float),
                                                   _ptr(avel, C.c_float), _ptr(ptype, C.c_uint),

@@ -231,10 +231,10 @@ class Ensemble:
         return _check(self.lib.blaze_ens_sync(self.h), "blaze_ens_sync")
 
     def state(self):
-        n = self.n
-        out = dict(pos=np.zeros((n, 3), np.float32), radius=np.zeros(n, np.float32),
-                   vel=np.zeros((n, 3), np.float32), avel=np.zeros((n, 3), np.float32),
-                   sys=np.zeros(n, np.int32), pid=np.zeros(n, np.int32))
+        n = self.n   # every entry is written by the library
+        out = dict(pos=np.empty((n, 3), np.float32), radius=np.empty(n, np.float32),
+                   vel=np.empty((n, 3), np.float32), avel=np.empty((n, 3), np.float32),
+                   sys=np.empty(n, np.int32), pid=np.empty(n, np.int32))
         st = _check(self.lib.blaze_ens_get_state(
             self.h, _ptr(out["pos"], C.c_float), _ptr(out["radius"], C.c_float),
             _ptr(out["vel"], C.c_float), _ptr(out["avel"], C.c_float),
@@ -344,7 +344,7 @@ class Adjoint:
         n = self.ens.n
         c = lambda a: None if a is None else np.ascontiguousarray(a, np.float32).reshape(n, 3)
         gpos, gvel, gavel = c(gpos), c(gvel), c(gavel)
-        out = [np.zeros((n, 3), np.float32) for _ in range(3)]
+        out = [np.empty((n, 3), np.float32) for _ in range(3)]
         gc = np.zeros((self.ens.nsys, 5), np.float64)
         ptrs = [_ptr(gpos, C.c_float), _ptr(gvel, C.c_float), _ptr(gavel, C.c_float)] + \
             [_ptr(a, C.c_float) for a in out] + [gc.ctypes.data_as(C.POINTER(C.c_double))]
