@@ -105,6 +105,21 @@ __device__ __forceinline__ bool list_needs_rebuild(float skin, const StepLink& l
   return false;
 }
 
+// Particles per warp of a step of n particles.  A warp shares its particles'
+// contacts among its lanes, so with fewer particles its chain of dependent
+// loads and laws is shorter; where full warps would not fill the GPU (148 SMs
+// of 24 warps) the particles are spread over more of them.
+inline int warp_particles(int n) {
+  int p = 32;
+  while (p > 4 && (n + p / 2 - 1) / (p / 2) <= 148 * 24) p /= 2;
+  return p;
+}
+// blocks of `threads` that hold n particles, wp to a warp
+inline int warp_blocks(int n, int wp, int threads) {
+  const int warps = (n + wp - 1) / wp, per = threads / 32;
+  return (warps + per - 1) / per;
+}
+
 struct WallGrid {       // per-cell candidate wall ops (CSR), optional
   const uint32_t* off;  // ncell_tab + 1 entries, or null = test every op
   const uint16_t* ops;
