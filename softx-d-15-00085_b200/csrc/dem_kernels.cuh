@@ -51,11 +51,22 @@ struct NbrList {
 // How a step learns whether it consumes a fresh re-sort, and how it asks for
 // the next one: through StepCtl (plain stepping) or, inside a CUDA graph,
 // through the IF-node condition of the next step.
+// An ensemble's round of steps (graph stepping): the steps of a round are
+// launched in a row, and a step does nothing when an earlier one of the round
+// has asked for a re-sort (k > *stop) or the call's steps are done (k >=
+// *left).
+struct RoundLink {
+  const int* left;   // steps still to run when the round began (null: not in a round)
+  int* stop;         // the first step of the round that asked for a re-sort
+  int k;             // this step's index in the round
+};
+
 struct StepLink {
   const int* rebuilt;                  // nonzero: read the sorted buffer
   cudaGraphConditionalHandle next_h;   // next step's IF condition (graph)
   int has_next_h;                      // 0: request through StepCtl::rebuild_req
   int check_next;                      // with a skin: the next step starts with a list check
+  RoundLink round;                     // ensembles
 };
 
 // With a Verlet skin the sphere and polyhedron paths run in blocks of

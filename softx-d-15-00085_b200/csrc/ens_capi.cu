@@ -69,9 +69,10 @@ struct blaze_ens {
   int* h_flags = nullptr;
   EnsCapture cap{};
   cudaStream_t stream = nullptr, aux = nullptr, aux2 = nullptr;
-  cudaGraphExec_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t graph[2] = {nullptr, nullptr};    // steps from S[c] (build_round_graph, build_if_graph)
   cudaGraphExec_t pgraph[2] = {nullptr, nullptr};   // persistent stepping, home S[c]
-  int* d_pw = nullptr;        // persistent stepping: left, done, req_step, barrier x3
+  int* d_pw = nullptr;        // persistent stepping: left, done, req_step, barrier x3; from 8 on
+                              // the rounds of graph stepping: left, stop, at, want
   float2* d_rot = nullptr;    // per system: (cos, sin) of the drum's turn so far
   bool any_rot = false;
   int persist_grid = 0;
@@ -441,12 +442,12 @@ int upload_params(blaze_ens* e) {
   return 0;
 }
 
-int enqueue_rebuild(blaze_ens* e, const int* gate, cudaStream_t st) {
+int enqueue_rebuild(blaze_ens* e, const int* gate, cudaStream_t st, const int* at = nullptr) {
   const int n = e->n;
   const EnsGeom g = geom(e);
-  ens_launch_hash(g, e->b, e->cur, n, e->cs, e->ctl, gate, st);
+  ens_launch_hash(g, e->b, e->cur, at, n, e->cs, e->ctl, gate, st);
   cell_scan_place(e->cs, n, &e->ctl->epoch, nullptr, gate, st);
-  ens_launch_reorder(e->b, e->cur, n, e->cs, e->ctl, gate, st);
+  ens_launch_reorder(e->b, e->cur, at, n, e->cs, e->ctl, gate, st);
   ens_launch_nlist(g, e->b, n, e->cs, e->ctl, gate, st);
   if (e->npoly > 0) {
     mix_launch_plist(g, e->b, mix_bufs(e), e->cs.start, e->ctl, gate, st);
@@ -466,7 +467,7 @@ int rebuild_kernel_count(const blaze_ens* e) {
 void launch_step_kernels(blaze_ens* e, StepLink link, cudaStream_t st,
                          const cudaEvent_t* ev = nullptr) {
   const EnsCapture* cap = e->opt.capture_forces ? &e->cap : nullptr;
-  if (e->npoly > 0) mix_launch_geom(mix_bufs(e), st);
+  if (e->npoly > 0) mix_launch_geom(mix_bufs(e), link.round, st);
   if (ev) cudaEventRecord(ev[0], st);
   if (e->npoly > 0) mix_launch_poly_step(geom(e), e->b, mix_bufs(e), e->cur, e->ctl, link, cap, st);
   if (ev) cudaEventRecord(ev[1], st);
@@ -485,7 +486,7 @@ int enqueue_step(blaze_ens* e) {
   if (rc) return rc;
   if (e->prof) CK(cudaEventRecord(e->pev[1], e->stream));
   launch_step_kernels(e, StepLink{&e->ctl->rebuilt, 0, 0}, e->stream, e->prof ? e->pev + 2 : nullptr);
-  if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, e->stream);
+  if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, RoundLink{}, e->stream);
   e->last_launches += 1 + step_kernel_count(e) + rebuild_kernel_count(e);
   e->cur ^= 1;
   if (e->prof) {   // re-sort, polyhedron geometry, polyhedron step, sphere step
@@ -500,10 +501,37 @@ int enqueue_step(blaze_ens* e) {
   return 0;
 }
 
+EnsRound round_words(const blaze_ens* e) {
+  return EnsRound{e->d_pw + 8, e->d_pw + 9, e->d_pw + 10, e->d_pw + 11};
+}
+
+// The conditional node (IF or WHILE) on h added to the graph being captured
+// on cs; its body in *body.
+int add_conditional(cudaStream_t cs, cudaGraphConditionalHandle h,
+                    cudaGraphConditionalNodeType type, cudaGraph_t* body) {
+  cudaStreamCaptureStatus status;
+  cudaGraph_t capg = nullptr;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t ndeps = 0;
+  CK(cudaStreamGetCaptureInfo(cs, &status, nullptr, &capg, &deps, &ndeps));
+  alignas(cudaGraphNodeParams) unsigned char raw[sizeof(cudaGraphNodeParams)];
+  std::memset(raw, 0, sizeof(raw));
+  cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(raw);
+  cp.type = cudaGraphNodeTypeConditional;
+  cp.conditional.handle = h;
+  cp.conditional.type = type;
+  cp.conditional.size = 1;
+  cudaGraphNode_t node;
+  CK(cudaGraphAddNode(&node, capg, deps, ndeps, &cp));
+  *body = cp.conditional.phGraph_out[0];
+  CK(cudaStreamUpdateCaptureDependencies(cs, &node, 1, cudaStreamSetCaptureDependencies));
+  return 0;
+}
+
 // kGraphSteps steps as one graph starting from S[c]: a gate kernel carries
 // the pending re-sort request into the first step's IF node; each step kernel
 // sets the next step's IF condition when any particle has moved half the skin.
-int build_graph(blaze_ens* e, int c) {
+int build_if_graph(blaze_ens* e, int c) {
   const int saved = e->cur;
   e->cur = c;
   cudaGraph_t g = nullptr;
@@ -515,35 +543,81 @@ int build_graph(blaze_ens* e, int c) {
                                    cudaStreamCaptureModeThreadLocal));
   launch_gate_graph(e->ctl, h[0], e->d_rb, kGraphSteps, e->stream);
   for (int k = 0; k < kGraphSteps; ++k) {
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t capg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(e->stream, &cs, nullptr, &capg, &deps, &ndeps));
-    alignas(cudaGraphNodeParams) unsigned char raw[sizeof(cudaGraphNodeParams)];
-    std::memset(raw, 0, sizeof(raw));
-    cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(raw);
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h[k];
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    CK(cudaGraphAddNode(&cnode, capg, deps, ndeps, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CK(cudaStreamUpdateCaptureDependencies(e->stream, &cnode, 1, cudaStreamSetCaptureDependencies));
+    cudaGraph_t body = nullptr;
+    int rc = add_conditional(e->stream, h[k], cudaGraphCondTypeIf, &body);
+    if (rc) return rc;
     CK(cudaStreamBeginCaptureToGraph(e->aux, body, nullptr, nullptr, 0,
                                      cudaStreamCaptureModeThreadLocal));
     CK(cudaMemsetAsync(e->d_rb + k, 0x01, sizeof(int), e->aux));
-    int rc = enqueue_rebuild(e, nullptr, e->aux);
+    rc = enqueue_rebuild(e, nullptr, e->aux);
     cudaGraph_t tmp = nullptr;
     CK(cudaStreamEndCapture(e->aux, &tmp));
     if (rc) return rc;
     const StepLink link = k + 1 < kGraphSteps ? StepLink{e->d_rb + k, h[k + 1], 1}
                                                : StepLink{e->d_rb + k, 0, 0};
     launch_step_kernels(e, link, e->stream);
-    if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, e->stream);
+    if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, RoundLink{}, e->stream);
     e->cur ^= 1;
   }
+  cudaGraph_t out = nullptr;
+  CK(cudaStreamEndCapture(e->stream, &out));
+  CK(cudaGraphInstantiate(&e->graph[c], out, 0));
+  CK(cudaGraphDestroy(out));
+  e->cur = saved;
+  return 0;
+}
+
+// Small ensembles (kRoundMax particles at most), from S[c]: one graph whose
+// WHILE node runs rounds until the call's steps are done
+// (ens_launch_round_init before each launch).  A round is a gate kernel, an IF
+// node with the re-sort when the round before asked for one, and kRoundSteps
+// steps in a row, of which those behind a step that asks for a re-sort do
+// nothing.  An IF node before every step costs about as much as a small step:
+// a box of 6,000 spheres, 16 steps, 171 us with IF nodes and a lane per
+// particle, 85 us in rounds with four particles to a warp.  The launches that
+// do nothing and the words that every step reads first cost a large ensemble
+// more than its IF nodes where the GPU has other work beside it: three hoppers
+// of 400,000 at once 2.77 against 2.66 ms a pass (one alone 3.91 against 4.08),
+// three mixed charges of 21,000 1.38 against 1.37.
+constexpr int kRoundSteps = 16;   // even: a whole round ends in the buffer it began in
+#ifndef BLAZE_ROUND_MAX
+#define BLAZE_ROUND_MAX 16384
+#endif
+constexpr int kRoundMax = BLAZE_ROUND_MAX;
+int build_round_graph(blaze_ens* e, int c) {
+  const int saved = e->cur;
+  const EnsRound r = round_words(e);
+  cudaGraph_t g = nullptr;
+  CK(cudaGraphCreate(&g, 0));
+  cudaGraphConditionalHandle hw;
+  CK(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
+  CK(cudaStreamBeginCaptureToGraph(e->stream, g, nullptr, nullptr, 0,
+                                   cudaStreamCaptureModeThreadLocal));
+  cudaGraph_t body = nullptr, ibody = nullptr, tmp = nullptr;
+  int rc = add_conditional(e->stream, hw, cudaGraphCondTypeWhile, &body);
+  if (rc) return rc;
+  cudaGraphConditionalHandle hi;
+  CK(cudaGraphConditionalHandleCreate(&hi, body, 0, 0));
+  CK(cudaStreamBeginCaptureToGraph(e->aux, body, nullptr, nullptr, 0,
+                                   cudaStreamCaptureModeThreadLocal));
+  ens_launch_round_gate(e->ctl, r, e->d_rb, hi, e->aux);
+  rc = add_conditional(e->aux, hi, cudaGraphCondTypeIf, &ibody);
+  if (rc) return rc;
+  CK(cudaStreamBeginCaptureToGraph(e->aux2, ibody, nullptr, nullptr, 0,
+                                   cudaStreamCaptureModeThreadLocal));
+  CK(cudaMemsetAsync(e->d_rb, 0x01, sizeof(int), e->aux2));
+  rc = enqueue_rebuild(e, nullptr, e->aux2, r.at);
+  CK(cudaStreamEndCapture(e->aux2, &tmp));
+  if (rc) return rc;
+  for (int k = 0; k < kRoundSteps; ++k) {
+    e->cur = c ^ (k & 1);
+    const RoundLink link{r.left, r.stop, k};
+    launch_step_kernels(e, StepLink{e->d_rb, 0, 0, 0, link}, e->aux);
+    if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, link, e->aux);
+  }
+  ens_launch_round_end(e->ctl, r, kRoundSteps, c, hw, e->aux);
+  CK(cudaStreamEndCapture(e->aux, &tmp));
+  ens_launch_round_last(e->b, r, e->n, e->stream);
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(e->stream, &out));
   CK(cudaGraphInstantiate(&e->graph[c], out, 0));
@@ -782,8 +856,8 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
   CKF(dalloc(&e->ctl, 1));
   CKF(dalloc(&e->d_rb, kGraphSteps));
   CKF(cudaMemset(e->d_rb, 0, sizeof(int) * kGraphSteps));
-  CKF(dalloc(&e->d_pw, 8));
-  CKF(cudaMemset(e->d_pw, 0, sizeof(int) * 8));
+  CKF(dalloc(&e->d_pw, 12));
+  CKF(cudaMemset(e->d_pw, 0, sizeof(int) * 12));
   CKF(dalloc(&e->d_rot, nsys));
   for (int s = 0; s < nsys; ++s) e->any_rot = e->any_rot || systems[s].rot_omega != 0.0f;
   {
@@ -960,12 +1034,16 @@ int blaze_ens_get_state(blaze_ens* e, float* pos3, float* radius, float* vel3, f
 
 namespace {
 
-// nsteps steps, as kGraphSteps-step CUDA graphs where `graphs` allows (the
-// remainder as plain steps).
+// nsteps steps, as CUDA graphs where `graphs` allows; what is left of a call
+// after its graphs, fewer than kGraphSteps steps, as plain steps (a round of
+// so few would mostly be launches that do nothing).
 int advance(blaze_ens* e, int nsteps, bool graphs) {
-  // persistent stepping (no drum turns: those advance between steps)
+  // persistent stepping (no drum turns: those advance between steps), where
+  // every particle has a lane of the resident grid; beyond that the step
+  // kernel's own grid is faster (400,000 spheres 121 against 105 us a step,
+  // boxes of 2,000,000 450 against 400)
   if (graphs && e->opt.use_graph == 2 && !e->opt.capture_forces && !e->any_rot && e->npoly == 0 &&
-      nsteps > 0) {
+      nsteps > 0 && e->n <= kEnsOneWave) {
     const int c = e->cur;
     if (!e->pgraph[c]) {
       int rc = build_persist_graph(e, c);
@@ -976,23 +1054,32 @@ int advance(blaze_ens* e, int nsteps, bool graphs) {
     e->last_launches += 3;   // the budget, then one round's gate and step kernels
     return 0;
   }
-  int done = 0;
-  while (done < nsteps) {
-    if (!graphs || nsteps - done < kGraphSteps) {
-      int rc = enqueue_step(e);
-      if (rc) return rc;
-      done += 1;
-      continue;
-    }
+  if (graphs && nsteps >= kGraphSteps && e->n <= kRoundMax) {
     const int c = e->cur;
     if (!e->graph[c]) {
-      int rc = build_graph(e, c);
+      int rc = build_round_graph(e, c);
+      if (rc) return rc;
+    }
+    ens_launch_round_init(round_words(e), nsteps, c, e->stream);
+    CK(cudaGraphLaunch(e->graph[c], e->stream));
+    const int rounds = (nsteps + kRoundSteps - 1) / kRoundSteps;   // with no re-sort
+    e->last_launches += 2 + rounds * (2 + kRoundSteps * step_kernel_count(e));
+    e->cur ^= nsteps & 1;
+    return 0;
+  }
+  for (; graphs && nsteps >= kGraphSteps; nsteps -= kGraphSteps) {
+    const int c = e->cur;
+    if (!e->graph[c]) {
+      int rc = build_if_graph(e, c);
       if (rc) return rc;
     }
     CK(cudaGraphLaunch(e->graph[c], e->stream));
     e->last_launches += 1 + kGraphSteps * step_kernel_count(e);
     if (kGraphSteps & 1) e->cur ^= 1;
-    done += kGraphSteps;
+  }
+  for (int k = 0; k < nsteps; ++k) {
+    int rc = enqueue_step(e);
+    if (rc) return rc;
   }
   CK(cudaGetLastError());
   return 0;

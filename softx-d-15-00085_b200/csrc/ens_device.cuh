@@ -13,6 +13,20 @@ __device__ __forceinline__ void ens_flag(StepCtl* ctl, uint32_t bits) {
   if (all && (threadIdx.x & 31) == (__ffs(m) - 1)) atomicOr(&ctl->status, all);
 }
 
+// Whether a step runs (always outside a round).
+__device__ __forceinline__ bool round_runs(const RoundLink& r) {
+  return !r.left || (r.k < *r.left && r.k <= *(volatile int*)r.stop);
+}
+__device__ __forceinline__ bool step_rebuilt(const StepLink& link) {
+  return (!link.round.left || link.round.k == 0) && *link.rebuilt != 0;
+}
+// Ask for a re-sort before the next step.
+__device__ __forceinline__ void request_resort(const StepLink& link, StepCtl* ctl) {
+  if (link.round.left) atomicMin(link.round.stop, link.round.k);
+  else if (link.has_next_h) cudaGraphSetConditional(link.next_h, 1u);
+  else atomicExch(&ctl->rebuild_req, 1);
+}
+
 __device__ __forceinline__ int3 ens_cell(const EnsSysDev& S, float3 p) {
   int3 c;
   c.x = (int)floorf((p.x - S.origin.x) / S.cell);

@@ -34,9 +34,12 @@ constexpr int kThreads = 256;
 
 // ------------------------------------------------------------------- hash
 __global__ void __launch_bounds__(kSortThreads)
-k_ens_hash(EnsGeom g, const float4* __restrict__ pos, const float4* __restrict__ vel, int n,
-           CellSort cs, StepCtl* ctl, const int* gate) {
+k_ens_hash(EnsGeom g, StateBuf s0, StateBuf s1, const int* at, int n, CellSort cs, StepCtl* ctl,
+           const int* gate) {
   if (gate && *gate == 0) return;
+  const bool second = at && *at != 0;
+  const float4* __restrict__ pos = second ? s1.pos : s0.pos;
+  const float4* __restrict__ vel = second ? s1.vel : s0.vel;
   const int i = blockIdx.x * kSortThreads + threadIdx.x;
   const bool valid = i < n;
   uint32_t st = 0, key = 0;
@@ -59,9 +62,10 @@ k_ens_hash(EnsGeom g, const float4* __restrict__ pos, const float4* __restrict__
 // (the place pass before it has already counted the re-sort: the old lists
 // are those of the other parity)
 __global__ void __launch_bounds__(kSortThreads)
-k_ens_reorder(StateBuf src, StateBuf dst, EnsBufs b, int n, CellSort cs, const StepCtl* ctl,
-              const int* gate) {
+k_ens_reorder(StateBuf s0, StateBuf s1, const int* at, StateBuf dst, EnsBufs b, int n, CellSort cs,
+              const StepCtl* ctl, const int* gate) {
   if (gate && *gate == 0) return;
+  const StateBuf src = at && *at != 0 ? s1 : s0;
   const int j = blockIdx.x * kSortThreads + threadIdx.x;
   const bool valid = j < n;
   const int i = cell_dest(cs, j, valid);
@@ -346,8 +350,8 @@ __device__ __forceinline__ float ens_particle_step_ref(const EnsGeom& g, const E
 // particle's first, every particle's second, ...), so that lanes side by
 // side mostly read and write the history of the same slot.  Wall contacts
 // (a few particles of a warp, for one wall after the other) go the same way.
-// Per 32 steps: hopper of 400,000 spheres 3.56 -> 2.84 ms, settled boxes of
-// 2,000,000 14.45 -> 13.96 ms, mixed charge of 21,000 1.67 -> 1.49 ms.
+// Per 32 steps: hopper of 400,000 spheres 3.56 -> 2.66 ms, settled boxes of
+// 2,000,000 14.0 -> 11.5 ms, mixed charge of 21,000 1.67 -> 1.49 ms.
 constexpr int kPairChunk = 96;     // pair contacts in shared memory at a time
 constexpr int kWallChunk = 64;     // wall contacts
 constexpr int kContactWords = 624; // shared words per warp
@@ -358,8 +362,8 @@ constexpr size_t contact_bytes(int threads) {
 }
 constexpr unsigned kAll = 0xffffffffu;
 
-// The step of particle i (every lane of a warp calls it with consecutive i;
-// valid: i < n): its contacts in list order (tangential histories updated in
+// The step of particle i (every lane of a warp calls it, the lanes of valid
+// particles first and with consecutive i): its contacts in list order (tangential histories updated in
 // place, the particle's own slots only), its walls, symplectic Euler from
 // `in` into `out`.  Raises status bits in st; returns the path
 // the particle has moved since the last re-sort.  kRecord: also writes what
@@ -431,7 +435,6 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     }
   }
   const int mine = __popc(cmask);
-  const int most = __reduce_max_sync(kAll, mine);
   const int total = __reduce_add_sync(kAll, mine);
   float* shf = reinterpret_cast<float*>(sh);
   uint16_t* con = reinterpret_cast<uint16_t*>(sh + 6 * kPairChunk);   // lane | slot << 5 | polyhedron << 14 | contact << 15
@@ -488,18 +491,29 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     L.hz[sk] = xi.z;
     return 0x8000u;
   };
+  // row m: every particle's contact of rank m; m0 the first row that reaches
+  // into the chunk, which starts at contact row0
+  int m0 = 0, row0 = 0;
   for (int c0 = 0; c0 < total; c0 += kPairChunk) {
     const int nc = min(kPairChunk, total - c0);
-    uint32_t cm = cmask;
-    for (int m = 0, row = -c0; m < most; ++m) {
+    int m1 = m0, row1 = row0;
+    uint32_t cm = cmask;   // this lane's contacts from row m on
+    uint32_t cm1 = cm;
+    for (int m = m0, row = row0 - c0; row < nc; ++m) {
       const unsigned bal = __ballot_sync(kAll, mine > m);
       if (mine > m) {
         const int c = row + __popc(bal & below);
-        if (c >= 0 && c < kPairChunk) con[c] = (uint16_t)(lane | (__ffs(cm) - 1) << 5);
+        if (c >= 0 && c < nc) con[c] = (uint16_t)(lane | (__ffs(cm) - 1) << 5);
         cm &= cm - 1u;
       }
       row += __popc(bal);
+      if (row <= nc) {
+        m1 = m + 1;
+        row1 = row + c0;
+        cm1 = cm;
+      }
     }
+    cmask = cm1;
     __syncwarp();
     for (int r0 = 0; r0 < nc; r0 += 32) {
       const int r = r0 + lane;
@@ -524,10 +538,10 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
       }
     }
     __syncwarp();
-    for (int m = 0, row = -c0; m < most; ++m) {
+    for (int m = m0, row = row0 - c0; row < nc; ++m) {
       const unsigned bal = __ballot_sync(kAll, mine > m);
       const int c = row + __popc(bal & below);
-      if (mine > m && c >= 0 && c < kPairChunk) {
+      if (mine > m && c >= 0 && c < nc) {
         const uint32_t v = con[c];
         if (v & 0x8000u) {
           f = f + f3(shf[c], shf[kPairChunk + c], shf[2 * kPairChunk + c]);
@@ -538,6 +552,8 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
       row += __popc(bal);
     }
     __syncwarp();
+    m0 = m1;
+    row0 = row1;
   }
   if (mask != mask_o) L.mask[i] = mask;
   if constexpr (kRecord) {
@@ -769,13 +785,19 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
 template <int kLaw, bool kCapture, bool kRecord, bool kCurved, bool kRot, bool kMix>
 __device__ __forceinline__ void ens_step_body(const EnsGeom& g, const EnsBufs& b,
                                               const StateBuf& in_plain, const StateBuf& in_sorted,
-                                              const StateBuf& out, int n, StepCtl* ctl,
+                                              const StateBuf& out, int n, int wp, StepCtl* ctl,
                                               const StepLink& link, const EnsCapture& cap,
                                               const EnsTape& tp) {
   extern __shared__ uint32_t contact_sh[];
-  const bool rebuilt = *link.rebuilt != 0;
+  if constexpr (!kRecord) {
+    if (!round_runs(link.round)) return;
+  }
+  const bool rebuilt = step_rebuilt(link);
   const StateBuf in = rebuilt ? in_sorted : in_plain;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // wp particles per warp (ens_warp_particles)
+  const int lane = threadIdx.x & 31;
+  const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wp + lane;
+  const bool valid = lane < wp && i < n;
   const int e = ctl->epoch & 1;
   const EnsList L = b.L[e];
   TapeView tv{};
@@ -784,47 +806,42 @@ __device__ __forceinline__ void ens_step_body(const EnsGeom& g, const EnsBufs& b
     const TapeStep ts = tp.steps[tp.ctl->slot];
     tv = tape_view(tp, ts.block, n);
     uint32_t words = 0;
-    if (i < n)
+    if (valid)
       words = 3u * (uint32_t)__popc(L.mask[i]) +
               4u * (uint32_t)__popc(__float_as_uint(in.vel[i].w) >> kSysBits);
     bool ok;
     const uint32_t off =
         tape_reserve(words, &tp.ctl->cur, tp.ctl->lim, ts.hbase, &tp.ctl->overflow, ok);
-    if (i < n) {
+    if (valid) {
       tv.hoff[i] = off;
       if (ok) hrec = reinterpret_cast<float*>(tp.arena + ts.hbase + off);
     }
   }
   uint32_t st = 0;
   const float path = ens_particle_step<kLaw, kCapture, kRecord, kCurved, true, kRot, kMix>(
-      g, b, in, out, i, i < n, e, L, tv, hrec, cap, st,
+      g, b, in, out, i, valid, e, L, tv, hrec, cap, st,
       contact_sh + (threadIdx.x >> 5) * kContactWords);
   {
     const unsigned m = __activemask();
     const unsigned req = __ballot_sync(m, path > 0.5f * g.skin);
-    if (req && (threadIdx.x & 31) == (__ffs(m) - 1)) {
-      if (link.has_next_h) cudaGraphSetConditional(link.next_h, 1u);
-      else atomicExch(&ctl->rebuild_req, 1);
-    }
+    if (req && (threadIdx.x & 31) == (__ffs(m) - 1)) request_resort(link, ctl);
   }
   ens_flag(ctl, st);
 }
 
 // Registers: 64 (four blocks of 256 per SM, with some spills) where the grid
 // has more blocks than the GPU holds, since the law's dependent chains need the
-// warps; 80 where it has fewer and the warps are there anyway (kOneWave, at
-// most kOneWave particles).  Per pass at 64, 80 and 96: settled boxes of
+// warps; 80 where it has fewer (kEnsOneWave particles at most).  Per pass at 64, 80 and 96: settled boxes of
 // 2,000,000 spheres, 32 steps, 13.9, 14.7, 17.4 ms; hopper of 400,000, 32 steps,
 // 2.85, 2.90, 3.26 ms; mixed charge of 21,000, 32 steps, 1.53, 1.49, 1.50 ms; a
 // box of 6,000, 16 steps, 181, 168, 166 us.
 constexpr int kStepRegs = 64, kStepRegsSmall = 80;
-constexpr int kOneWave = 148 * 3 * 256;
 template <int kLaw, bool kCapture, bool kCurved, bool kRot, bool kMix, bool kSmall>
 __global__ void __maxnreg__(kSmall ? kStepRegsSmall : kStepRegs)
 k_ens_step(EnsGeom g, EnsBufs b, StateBuf in_plain, StateBuf in_sorted, StateBuf out, int n,
-           StepCtl* ctl, StepLink link, EnsCapture cap) {
-  ens_step_body<kLaw, kCapture, false, kCurved, kRot, kMix>(g, b, in_plain, in_sorted, out, n, ctl,
-                                                           link, cap, EnsTape{});
+           int wp, StepCtl* ctl, StepLink link, EnsCapture cap) {
+  ens_step_body<kLaw, kCapture, false, kCurved, kRot, kMix>(g, b, in_plain, in_sorted, out, n, wp,
+                                                           ctl, link, cap, EnsTape{});
 }
 
 // The recording step (reverse mode, linear law, plane walls) held to the
@@ -833,13 +850,15 @@ k_ens_step(EnsGeom g, EnsBufs b, StateBuf in_plain, StateBuf in_sorted, StateBuf
 constexpr int kRecordRegs = 80;
 __global__ void __maxnreg__(kRecordRegs)
 k_ens_step_rec(EnsGeom g, EnsBufs b, StateBuf in_plain, StateBuf in_sorted, StateBuf out, int n,
-               StepCtl* ctl, StepLink link, EnsTape tp) {
+               int wp, StepCtl* ctl, StepLink link, EnsTape tp) {
   ens_step_body<kLawLinear, false, true, false, false, false>(
-      g, b, in_plain, in_sorted, out, n, ctl, link, EnsCapture{nullptr, nullptr}, tp);
+      g, b, in_plain, in_sorted, out, n, wp, ctl, link, EnsCapture{nullptr, nullptr}, tp);
 }
 
 // ------------------------------------------------------------ drum turn
-__global__ void k_ens_rot_tick(const EnsSysDev* __restrict__ sys, float2* rot, int nsys) {
+__global__ void k_ens_rot_tick(const EnsSysDev* __restrict__ sys, float2* rot, int nsys,
+                               RoundLink round) {
+  if (!round_runs(round)) return;
   const int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nsys || !sys[s].rot) return;
   const float2 r = rot[s];
@@ -847,6 +866,46 @@ __global__ void k_ens_rot_tick(const EnsSysDev* __restrict__ sys, float2* rot, i
   const float s1 = r.y * sys[s].rot_cd + r.x * sys[s].rot_sd;
   const float m = sqrtf(c1 * c1 + s1 * s1);
   rot[s] = make_float2(c1 / m, s1 / m);
+}
+
+// ---------------------------------------------------------------- rounds
+__global__ void k_round_init(EnsRound r, int steps, int at) {
+  *r.left = steps;
+  *r.at = at;
+  *r.want = at ^ (steps & 1);
+}
+
+__global__ void k_round_gate(StepCtl* ctl, EnsRound r, int* rb, cudaGraphConditionalHandle if_h) {
+  const int req = ctl->rebuild_req;
+  ctl->rebuild_req = 0;
+  *rb = 0;
+  *r.stop = 0x7fffffff;
+  cudaGraphSetConditional(if_h, req ? 1u : 0u);
+}
+
+__global__ void k_round_end(StepCtl* ctl, EnsRound r, int steps, int home,
+                            cudaGraphConditionalHandle loop_h) {
+  int ran = min(steps, *r.left);
+  if (*r.stop < ran) {
+    ran = *r.stop + 1;
+    ctl->rebuild_req = 1;
+  }
+  const int left = *r.left - ran;
+  *r.left = left;
+  *r.at = home ^ (ran & 1);
+  cudaGraphSetConditional(loop_h, left > 0 ? 1u : 0u);
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_round_last(StateBuf s0, StateBuf s1, EnsRound r, int n) {
+  const int at = *r.at;
+  if (at == *r.want) return;
+  const StateBuf src = at ? s1 : s0, dst = at ? s0 : s1;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  dst.pos[i] = src.pos[i];
+  dst.vel[i] = src.vel[i];
+  dst.angv[i] = src.angv[i];
 }
 
 // ------------------------------------------------------- persistent steps
@@ -920,15 +979,16 @@ __global__ void k_barrier_check(unsigned int* bar, StepCtl* ctl) {
 
 template <int kLaw, bool kCurved>
 __global__ void __maxnreg__(kPersistRegs)
-k_ens_persist(EnsGeom g, EnsBufs b, StateBuf home, StateBuf other, StateBuf sorted, int n,
+k_ens_persist(EnsGeom g, EnsBufs b, StateBuf home, StateBuf other, StateBuf sorted, int n, int wp,
               StepCtl* ctl, const int* rebuilt, EnsPersist p) {
   extern __shared__ uint32_t contact_sh[];
   const int e = ctl->epoch & 1;
   const EnsList L = b.L[e];
   const int budget = *p.left;
   const bool rb = *rebuilt != 0;
-  const int gstride = gridDim.x * blockDim.x;
-  const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int gstride = (int)(gridDim.x * (blockDim.x >> 5)) * wp;
+  const int i0 = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * wp + lane;
   int done = 0;
   bool stop = false, aborted = false;
   for (int k = 0; k < budget && !stop; ++k) {
@@ -936,9 +996,9 @@ k_ens_persist(EnsGeom g, EnsBufs b, StateBuf home, StateBuf other, StateBuf sort
     const StateBuf out = (k & 1) ? home : other;
     uint32_t st = 0;
     bool req = false;
-    for (int i = i0; i - (int)(threadIdx.x & 31) < n; i += gstride) {   // whole warps
+    for (int i = i0; i - lane < n; i += gstride) {   // whole warps
       const float path = ens_particle_step<kLaw, false, false, kCurved, false>(
-          g, b, in, out, i, i < n, e, L, TapeView{}, nullptr, EnsCapture{nullptr, nullptr}, st,
+          g, b, in, out, i, lane < wp && i < n, e, L, TapeView{}, nullptr, EnsCapture{nullptr, nullptr}, st,
           contact_sh + (threadIdx.x >> 5) * kContactWords);
       req |= path > 0.5f * g.skin;
     }
@@ -949,7 +1009,8 @@ k_ens_persist(EnsGeom g, EnsBufs b, StateBuf home, StateBuf other, StateBuf sort
     stop = *(volatile int*)p.req_step <= k;
   }
   if (!aborted && (done & 1)) {
-    for (int i = i0; i < n; i += gstride) {
+    for (int i = (int)(blockIdx.x * blockDim.x + threadIdx.x); i < n;
+         i += (int)(gridDim.x * blockDim.x)) {
       home.pos[i] = other.pos[i];
       home.vel[i] = other.vel[i];
       home.angv[i] = other.angv[i];
@@ -1022,15 +1083,16 @@ inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
 
 }  // namespace
 
-void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, const CellSort& cs,
-                     StepCtl* ctl, const int* gate, cudaStream_t st) {
-  k_ens_hash<<<sort_blocks(n), kSortThreads, 0, st>>>(g, b.S[cur].pos, b.S[cur].vel, n, cs, ctl,
-                                                      gate);
+void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, const int* at, int n,
+                     const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st) {
+  k_ens_hash<<<sort_blocks(n), kSortThreads, 0, st>>>(g, b.S[at ? 0 : cur], b.S[1], at, n, cs,
+                                                      ctl, gate);
 }
 
-void ens_launch_reorder(const EnsBufs& b, int cur, int n, const CellSort& cs, StepCtl* ctl,
-                        const int* gate, cudaStream_t st) {
-  k_ens_reorder<<<sort_blocks(n), kSortThreads, 0, st>>>(b.S[cur], b.S[2], b, n, cs, ctl, gate);
+void ens_launch_reorder(const EnsBufs& b, int cur, const int* at, int n, const CellSort& cs,
+                        StepCtl* ctl, const int* gate, cudaStream_t st) {
+  k_ens_reorder<<<sort_blocks(n), kSortThreads, 0, st>>>(b.S[at ? 0 : cur], b.S[1], at, b.S[2],
+                                                         b, n, cs, ctl, gate);
 }
 
 void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const CellSort& cs, StepCtl* ctl,
@@ -1043,11 +1105,12 @@ void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl
                      StepLink link, const EnsCapture* cap, int block, cudaStream_t st) {
   const EnsCapture c = cap ? *cap : EnsCapture{nullptr, nullptr};
   const int bs = block >= 64 && block <= kMaxStepBlock && block % 32 == 0 ? block : kThreads;
-  const int gs = (n + bs - 1) / bs;
-#define ENS_ARGS g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, ctl, link, c
+  const int wp = ens_warp_particles(g.law, n);
+  const int gs = warp_blocks(n, wp, bs);
+#define ENS_ARGS g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, wp, ctl, link, c
 #define ENS_LAUNCH(...)                                                             \
   do {                                                                              \
-    if (n <= kOneWave)                                                              \
+    if (n <= kEnsOneWave)                                                              \
       k_ens_step<__VA_ARGS__, true><<<gs, bs, contact_bytes(bs), st>>>(ENS_ARGS);   \
     else                                                                            \
       k_ens_step<__VA_ARGS__, false><<<gs, bs, contact_bytes(bs), st>>>(ENS_ARGS);  \
@@ -1104,9 +1167,10 @@ void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl
 void ens_launch_step_record(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl* ctl,
                             StepLink link, const EnsTape& tape, int block, cudaStream_t st) {
   const int bs = block >= 64 && block <= kMaxStepBlock && block % 32 == 0 ? block : kThreads;
-  const int gs = (n + bs - 1) / bs;
+  const int wp = ens_warp_particles(g.law, n);
+  const int gs = warp_blocks(n, wp, bs);
   // reverse mode accepts plane walls only (blaze_ens_adj_create)
-  k_ens_step_rec<<<gs, bs, contact_bytes(bs), st>>>(g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, ctl, link, tape);
+  k_ens_step_rec<<<gs, bs, contact_bytes(bs), st>>>(g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, wp, ctl, link, tape);
 }
 
 int ens_persist_grid(const EnsGeom& g, int block, int n) {
@@ -1125,7 +1189,7 @@ int ens_persist_grid(const EnsGeom& g, int block, int n) {
               ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_persist<kLawHertz, false>, block, contact_bytes(block))
               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_persist<kLawLinear, false>, block, contact_bytes(block));
   if (err != cudaSuccess || per_sm < 1) return 0;
-  const int need = (n + block - 1) / block;
+  const int need = warp_blocks(n, ens_warp_particles(g.law, n), block);
   return std::max(1, std::min(need, per_sm * sms));
 }
 
@@ -1144,19 +1208,37 @@ cudaError_t ens_launch_persist(const EnsGeom& g, const EnsBufs& b, int home, int
   cfg.numAttrs = coop ? 1 : 0;
   const StateBuf sh = b.S[home], so = b.S[home ^ 1], ss = b.S[2];
   if (g.law == kLawReference)
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawReference, false>, g, b, sh, so, ss, n, ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawReference, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
   if (g.curved) {
     if (g.law == kLawHertz)
-      return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, true>, g, b, sh, so, ss, n, ctl, rebuilt, p);
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, true>, g, b, sh, so, ss, n, ctl, rebuilt, p);
+      return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, true>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, true>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
   }
   if (g.law == kLawHertz)
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, false>, g, b, sh, so, ss, n, ctl, rebuilt, p);
-  return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, false>, g, b, sh, so, ss, n, ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
+  return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
 }
 
-void ens_launch_rot_tick(const EnsGeom& g, int nsys, cudaStream_t st) {
-  k_ens_rot_tick<<<(nsys + kThreads - 1) / kThreads, kThreads, 0, st>>>(g.sys, g.rot, nsys);
+void ens_launch_rot_tick(const EnsGeom& g, int nsys, const RoundLink& round, cudaStream_t st) {
+  k_ens_rot_tick<<<(nsys + kThreads - 1) / kThreads, kThreads, 0, st>>>(g.sys, g.rot, nsys, round);
+}
+
+void ens_launch_round_init(const EnsRound& r, int steps, int at, cudaStream_t st) {
+  k_round_init<<<1, 1, 0, st>>>(r, steps, at);
+}
+
+void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb,
+                           cudaGraphConditionalHandle if_h, cudaStream_t st) {
+  k_round_gate<<<1, 1, 0, st>>>(ctl, r, rb, if_h);
+}
+
+void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int steps, int home,
+                          cudaGraphConditionalHandle loop_h, cudaStream_t st) {
+  k_round_end<<<1, 1, 0, st>>>(ctl, r, steps, home, loop_h);
+}
+
+void ens_launch_round_last(const EnsBufs& b, const EnsRound& r, int n, cudaStream_t st) {
+  k_round_last<<<nblk(n), kThreads, 0, st>>>(b.S[0], b.S[1], r, n);
 }
 
 void ens_launch_barrier_check(unsigned int* bar, StepCtl* ctl, cudaStream_t st) {

@@ -297,13 +297,19 @@ __device__ __forceinline__ uint32_t tape_reserve(uint32_t words, unsigned long l
 }
 
 // One re-sort: hash (key and count), cell_scan_place on &ctl->epoch, reorder,
-// nlist.
-void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, int n, const CellSort& cs,
-                     StepCtl* ctl, const int* gate, cudaStream_t st);
-void ens_launch_reorder(const EnsBufs& b, int cur, int n, const CellSort& cs, StepCtl* ctl,
-                        const int* gate, cudaStream_t st);
+// nlist.  The state is in S[cur], or in S[*at] when at is given.
+void ens_launch_hash(const EnsGeom& g, const EnsBufs& b, int cur, const int* at, int n,
+                     const CellSort& cs, StepCtl* ctl, const int* gate, cudaStream_t st);
+void ens_launch_reorder(const EnsBufs& b, int cur, const int* at, int n, const CellSort& cs,
+                        StepCtl* ctl, const int* gate, cudaStream_t st);
 void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const CellSort& cs, StepCtl* ctl,
                       const int* gate, cudaStream_t st);
+// Particles per warp (warp_particles); the reference law walks a particle's
+// contacts on its own lane.
+inline int ens_warp_particles(int law, int n) { return law == kLawReference ? 32 : warp_particles(n); }
+// particles that the step's resident grid holds, a lane each (148 SMs, three
+// blocks of 256)
+constexpr int kEnsOneWave = 148 * 3 * 256;
 // `block`: threads per block (64 .. kMaxStepBlock, a multiple of 32).
 constexpr int kMaxStepBlock = 512;
 void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl* ctl,
@@ -314,7 +320,23 @@ void ens_launch_step_record(const EnsGeom& g, const EnsBufs& b, int cur, int n, 
                             StepLink link, const EnsTape& tape, int block, cudaStream_t st);
 // After a step: every turning system's (cos, sin) advanced by its increment
 // and renormalised.
-void ens_launch_rot_tick(const EnsGeom& g, int nsys, cudaStream_t st);
+void ens_launch_rot_tick(const EnsGeom& g, int nsys, const RoundLink& round, cudaStream_t st);
+// Rounds of steps (RoundLink).  Before a call's first round (init): its steps
+// and the buffer S[at] it starts from.  At a round's start (gate): the pending
+// re-sort request into the IF node, *rb = 0.  Every round's steps are launched
+// as if its state were in S[home] (a re-sort's copy is read instead by the
+// first); a round that runs to its end leaves it there, and one that stops
+// early is followed by a re-sort, which reads S[*r.at].  At its end: the steps
+// it ran off *left, loop_h (the WHILE node around the rounds) set while some
+// are left.  After the last (last): the state copied to S[*r.want], where the
+// host expects it after an even or odd number of steps, if it is not there.
+struct EnsRound { int* left; int* stop; int* at; int* want; };
+void ens_launch_round_init(const EnsRound& r, int steps, int at, cudaStream_t st);
+void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb,
+                           cudaGraphConditionalHandle if_h, cudaStream_t st);
+void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int steps, int home,
+                          cudaGraphConditionalHandle loop_h, cudaStream_t st);
+void ens_launch_round_last(const EnsBufs& b, const EnsRound& r, int n, cudaStream_t st);
 // Persistent stepping: one cooperative launch runs up to *left steps with a
 // grid barrier between steps and returns at the first step that asks for a
 // re-sort (ctl->rebuild_req set) or when the budget is spent, with the state

@@ -41,7 +41,8 @@ k_mix_mark(StateBuf s, MixBufs m, const int* __restrict__ caller_index,
 // -------------------------------------------------------------- geometry
 // One thread per (polyhedron, vertex or face).
 __global__ void __launch_bounds__(kThreads)
-k_mix_geom(MixBufs m) {
+k_mix_geom(MixBufs m, RoundLink round) {
+  if (!round_runs(round)) return;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int p = t / (kMixMaxV + kMixMaxF), item = t % (kMixMaxV + kMixMaxF);
   if (p >= m.npoly) return;
@@ -388,7 +389,8 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
   __shared__ MixSmem sm;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int p = blockIdx.x;
-  const bool rebuilt = *link.rebuilt != 0;
+  if (!round_runs(link.round)) return;
+  const bool rebuilt = step_rebuilt(link);
   const StateBuf in = rebuilt ? in_sorted : in_plain;
   const int e = ctl->epoch & 1;
   const MixList L = m.L[e];
@@ -802,10 +804,7 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
       cap.f[i] = make_float4(f.x, f.y, f.z, 0.0f);
       cap.t[i] = make_float4(t.x, t.y, t.z, 0.0f);
     }
-    if (path > 0.5f * g.skin) {
-      if (link.has_next_h) cudaGraphSetConditional(link.next_h, 1u);
-      else atomicExch(&ctl->rebuild_req, 1);
-    }
+    if (path > 0.5f * g.skin) request_resort(link, ctl);
   }
   st = __reduce_or_sync(0xffffffffu, st);
   if (lane == 0 && st) atomicOr(&ctl->status, st);
@@ -819,9 +818,9 @@ void mix_launch_mark(const EnsBufs& b, int cur, const MixBufs& m, const int* cal
   k_mix_mark<<<nblk(m.npoly), kThreads, 0, st>>>(b.S[cur], m, caller_index, quat);
 }
 
-void mix_launch_geom(const MixBufs& m, cudaStream_t st) {
+void mix_launch_geom(const MixBufs& m, const RoundLink& round, cudaStream_t st) {
   if (m.npoly <= 0) return;
-  k_mix_geom<<<nblk(m.npoly * (kMixMaxV + kMixMaxF)), kThreads, 0, st>>>(m);
+  k_mix_geom<<<nblk(m.npoly * (kMixMaxV + kMixMaxF)), kThreads, 0, st>>>(m, round);
 }
 
 void mix_launch_plist(const EnsGeom& g, const EnsBufs& b, const MixBufs& m,

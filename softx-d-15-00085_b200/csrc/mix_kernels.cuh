@@ -28,7 +28,7 @@ namespace blaze {
 // orientation, memory position, path and both list copies cleared.
 void mix_launch_mark(const EnsBufs& b, int cur, const MixBufs& m, const int* caller_index,
                      const float4* quat, cudaStream_t st);
-void mix_launch_geom(const MixBufs& m, cudaStream_t st);
+void mix_launch_geom(const MixBufs& m, const RoundLink& round, cudaStream_t st);
 void mix_launch_plist(const EnsGeom& g, const EnsBufs& b, const MixBufs& m,
                       const uint32_t* start, StepCtl* ctl,
                       const int* gate, cudaStream_t st);
