@@ -1,0 +1,175 @@
+"""The step kernels at the sizes where their launch changes: how many particles
+a warp takes (it shares its contacts among its lanes), rounds or IF nodes in
+graph stepping, persistent stepping's resident grid, the block sums of the
+energy tallies and the lifters' turn in the step's last block, and the windows
+of candidate triangles of a polyhedron.  Spheres against the FP32 restatements
+bit for bit (the energy sums are FP64 sums of at most some 5e5 terms of one
+sign in another order: within 5e5 x 2^-53 < 1e-10), stepping modes against each other bit for bit."""
+import math
+
+import numpy as np
+import pytest
+
+from bindings import EnsRestated, Restated
+from blaze import device, synth
+from blaze import ensemble as E
+from blaze import types as T
+
+pytestmark = pytest.mark.gpu
+
+
+def lattice(n, pitch, origin, seed):
+    """The first n sites of a cubic lattice, random order, jittered; and its side."""
+    rng = np.random.default_rng(seed)
+    m = int(math.ceil(n ** (1.0 / 3.0)))
+    g = np.arange(m ** 3)[:n]
+    p = np.stack([g % m, g // m % m, g // (m * m)], 1) * pitch + origin
+    p = p + rng.uniform(-1e-4, 1e-4, p.shape)
+    return p[rng.permutation(n)].astype(np.float32), rng, m * pitch
+
+
+@pytest.mark.parametrize("energy", [False, True])
+@pytest.mark.parametrize("n", [1, 33, 257, 14208, 14209, 28417, 56832, 56833])
+def test_sphere_step_sizes(tmp_path, n, energy):
+    if energy and n not in (257, 14209, 56833):
+        pytest.skip("the tallies' block sums: one size below and above a block, and many blocks")
+    r = 0.1
+    P, _ = synth.box_project(str(tmp_path), n_side=(2, 2, 2), radius=r)
+    P.sim_info.Num_Particles = n
+    P.sim_info.EnergyCalc = energy
+    pos, rng, _ = lattice(n, 0.1995, 0.0995, n)       # touching the walls and each other
+    vel = rng.normal(scale=10.0, size=(n, 3)).astype(np.float32)
+    avel = rng.normal(scale=30.0, size=(n, 3)).astype(np.float32)
+    ty, pid = np.zeros(n, np.uint32), np.arange(n, dtype=np.int32)
+    ref = Restated("f32").init(P.sim_info, P.wobj, P.n_w, P.pobj, P.n_p, P.dobj, P.n_d)
+    ref.set_state(pos, vel, avel, ty, pid)
+    sims = [device.Simulation(P, use_graph=g) for g in (0, 1)]
+    for s in sims:
+        s.set_state(pos, vel, avel, ty, pid)
+        s.step(1)
+        s.step(2)
+    ref.step(3)
+    want = ref.state()
+    for s in sims:
+        got = s.state()
+        assert got["status"] == 0
+        for k in ("pos", "vel", "avel"):
+            np.testing.assert_array_equal(got[k].astype(np.float64), want[k], err_msg=k)
+        np.testing.assert_array_equal(got["pid"], want["pid"])
+        if energy:
+            e, w = s.energy(), np.asarray(ref.energy(), np.float64)
+            assert e[0] > 0 and e[2] > 0
+            np.testing.assert_allclose(e, w, rtol=1e-10)
+    np.testing.assert_array_equal(sims[0].energy(), sims[1].energy())
+    for s in sims:
+        s.close()
+
+
+def ens_box(n):
+    """One box system in contact, hot enough to re-sort every few steps."""
+    r = 0.2
+    pos, rng, side = lattice(n, 0.4 - 2e-4, 0.2, n)
+    L, H = side + 0.02, 1.5 * side + 1.0
+    cell = 2.0 * r + 0.05
+    S = synth.box_system(n, L, H, cell, 0, density=2500e-6, kn=1e5, restitution=0.6, mu=0.4)
+    vel = rng.normal(scale=60.0, size=(n, 3)).astype(np.float32)
+    return [S], synth.box_walls(L, H), pos, np.full(n, r, np.float32), vel
+
+
+@pytest.mark.parametrize("n", [1, 3, 33, 14208, 14209, 16384, 16385, 28417, 56833, 113664, 113665])
+def test_ensemble_step_sizes(n):
+    """Calls of odd and even lengths end in either buffer; a round of 16 steps
+    stops early at every re-sort."""
+    S, W, pos, rad, vel = ens_box(n)
+    calls = (20, 9, 16, 3)
+    opt = dict(law=E.LAW_LINEAR, dt=5e-6, skin=0.02)
+    out, rb = [], []
+    for g in (0, 1, 2):
+        e = E.Ensemble(S, W, use_graph=g, **opt)
+        e.set_state(pos, rad, vel)
+        for c in calls:
+            e.step(c)
+        out.append(e.state())
+        rb.append(e.num_rebuilds())
+        e.close()
+    if n <= 16385:
+        o = EnsRestated(S, W, E.LAW_LINEAR, 5e-6, 0.02, 32, precision="f32")
+        o.set_state(pos, rad, vel)
+        o.step(sum(calls))
+        out.append(o.state())
+        rb.append(o.num_rebuilds())
+    assert out[0]["status"] == 0 and len(set(rb)) == 1
+    if n > 1000:
+        assert rb[0] > 2
+    for other in out[1:]:
+        for k in ("pos", "vel", "avel"):
+            np.testing.assert_array_equal(out[0][k].astype(np.float64), other[k].astype(np.float64), err_msg=k)
+        np.testing.assert_array_equal(out[0]["pid"], other["pid"])
+
+
+def test_mill_graph_equals_plain(tmp_path):
+    """Twelve blocks: lifters turned by the last block of the step before
+    (graphs) or by a kernel of their own, energy summed block by block."""
+    P, st = synth.mill_project(str(tmp_path), n=3000)
+    axis = float(P.wobj[0].cyl_geo.radius)
+    out = []
+    for g in (0, 1):
+        s = device.Simulation(P, skin=0.05, use_graph=g)
+        s.set_cylinder_rotation(True)
+        s.set_state(st["pos"], st["vel"], st["avel"], st["type"], st["pid"])
+        s.set_dobj_rotation(axis, axis, 50.0 * float(P.mill.RadPerStep))
+        for c in (19, 40, 8):
+            s.step(c)
+        d = s.dobj()
+        verts = [(v.x, v.y, v.z) for k in range(P.n_d) for v in d[k].vertex]
+        faces = [(f.normal.x, f.normal.y, f.centroid.x, f.centroid.y, f.area)
+                 for k in range(P.n_d) for f in d[k].faces]
+        out.append((s.state(), s.energy(), np.array(verts), np.array(faces)))
+        s.close()
+    (a, ea, va, fa), (b, eb, vb, fb) = out
+    for k in ("pos", "vel", "avel", "pid"):
+        np.testing.assert_array_equal(a[k], b[k], err_msg=k)
+    assert ea[0] > 0
+    np.testing.assert_array_equal(ea, eb)
+    np.testing.assert_array_equal(va, vb)
+    np.testing.assert_array_equal(fa, fb)
+    turned = abs(67 * 50.0 * float(P.mill.RadPerStep))
+    v0 = np.array([P.dobj[0].vertex[0].x - axis, P.dobj[0].vertex[0].y - axis])
+    v1 = va[0, :2] - axis
+    got = math.atan2(v0[0] * v1[1] - v0[1] * v1[0], v0 @ v1)
+    assert abs(abs(got) - turned) < 1e-3 * turned + 1e-5
+
+
+@pytest.mark.parametrize("side", [0.4, 1.1, 8.0])
+def test_polyhedra_on_a_fine_mesh(side):
+    """Rocks thrown on a floor of triangles: more than one window of candidate
+    triangles per rock (side 0.4 cm), about one, and two in all."""
+    S, _, p, r, sh, so, q = synth.mixed_box_ensemble(n_spheres=40, n_rocks=12, L=8.0, H=14.0, kn=1e5)
+    L, H = 8.0, 14.0
+    W = [w for k, w in enumerate(synth.box_walls(L, H)) if k != 4]
+    m = int(math.ceil(L / side))
+    x = np.linspace(0.0, L, m + 1)
+    for i in range(m):
+        for j in range(m):
+            a, b = (x[i], x[j], 0.0), (x[i + 1], x[j], 0.0)
+            c, d = (x[i + 1], x[j + 1], 0.0), (x[i], x[j + 1], 0.0)
+            W += [E.triangle(a, b, c), E.triangle(a, c, d)]
+    s = S[0]
+    s.nwalls, s.tri0, s.ntris = 5, 5, len(W) - 5
+    vel = np.zeros_like(p)
+    vel[:, 2] = -60.0
+    ens = E.Ensemble(S, W, law=E.LAW_LINEAR, dt=1e-5, skin=0.04, use_graph=1)
+    o = EnsRestated(S, W, E.LAW_LINEAR, 1e-5, 0.04, 32, precision="f32")
+    for e in (ens, o):
+        e.set_state(p, r, vel)
+        e.set_polyhedra(sh, so, q)
+        e.step(1600)
+    a, b = ens.state(), o.state()
+    assert a["status"] == b["status"] == 0
+    for k in ("pos", "vel", "avel"):
+        np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
+    np.testing.assert_array_equal(ens.orientations().astype(np.float64), o.orientations())
+    rocks = so[a["pid"]] >= 0
+    assert (a["vel"][rocks, 2] > 0).any()            # some have bounced
+    ens.close()
+    o.close()
