@@ -1188,7 +1188,7 @@ int blaze_ens_last_launches(blaze_ens* e) { return e ? e->last_launches : -1; }
 int blaze_ens_rebuild_kernels(blaze_ens* e) {
   if (!e) return -1;
   // persistent stepping: a re-sort also starts another round (gate + step)
-  return rebuild_kernel_count(e) + (e->opt.use_graph == 2 ? 2 : 0);
+  return rebuild_kernel_count(e) + (e->opt.use_graph == 2 && e->n <= kEnsOneWave ? 2 : 0);
 }
 
 }  // extern "C"
@@ -1653,7 +1653,7 @@ int restore_checkpoint(blaze_ens_adj* a, const EnsCheckpoint& c) {
 }
 
 // kGraphSteps recorded steps as one graph from S[c]: the step graph of
-// build_graph, with the list recorded inside each step's IF node (a
+// build_if_graph, with the list recorded inside each step's IF node (a
 // re-sort), then the tape tick and the recording step.
 int build_record_graph(blaze_ens_adj* a, int c) {
   blaze_ens* e = a->e;

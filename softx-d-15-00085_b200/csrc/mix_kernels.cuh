@@ -4,13 +4,13 @@
 // Per step, before the sphere step k_ens_step:
 //   k_mix_geom        world-frame vertex offsets and face planes of every
 //                     polyhedron from its orientation (FP64)
-//   k_mix_poly_step   one warp per polyhedron: sphere neighbours a slot per
-//                     lane (the pair's force and torque on the sphere left in
-//                     the slot for the sphere step), polyhedron neighbours one
-//                     pair at a time with the warp sharing the separating-axis
-//                     queries, walls a candidate triangle per lane; then lane 0
-//                     sums in slot order and integrates (translation, Euler's
-//                     equations in the body frame, quaternion)
+//   k_mix_poly_step   four warps per polyhedron that take its tests in turn:
+//                     sphere neighbours a slot per lane (the pair's force and
+//                     torque on the sphere left in the slot for the sphere
+//                     step), polyhedron neighbours and near triangles one at a
+//                     time with a warp sharing the separating-axis queries; then
+//                     one warp sums in slot order and integrates (translation,
+//                     Euler's equations in the body frame, quaternion)
 // and per re-sort, after the sphere list:
 //   k_mix_plist       the 64-slot neighbour list of every polyhedron, its
 //                     tangential histories carried by partner pid
