@@ -151,23 +151,33 @@ __device__ __forceinline__ float2 cell_gap(float p, float o, float cell, int g, 
 // (P. Markstein, IBM J. Res. Dev. 34(1), 1990; J.-M. Muller et al.,
 // Handbook of Floating-Point Arithmetic: with y within half an ulp of 1/b
 // and q1 within an ulp of a/b, the corrected quotient is correctly rounded,
-// barring underflow or overflow of the intermediate values).  A zero
-// numerator keeps its sign.  Outside the range where every intermediate is
-// normal and finite (b in [1e-15, 1e15], |a| in [1e-20, 1e15]: quotients
-// between 1e-35 and 1e30) the IEEE division is used.  blaze_check_division
-// compares it with IEEE division on the GPU.
+// barring underflow or overflow of the intermediate values).  A zero remainder
+// leaves the quotient as it is; a zero numerator gives zero, its sign set at
+// the end (b is positive: the quotient's sign is the numerator's).  Outside the
+// range where every intermediate is normal and finite (b in [1e-15, 1e15], every
+// |a| zero or in [1e-20, 1e15]: quotients between 1e-35 and 1e30) all three are
+// IEEE divisions.  The range is tested once, on the components' bits (those of
+// a zero less one wrap to the largest word; those of a NaN are above the limit):
+// with a test and two selects for each component a step of 100,000 spheres in
+// the reference's arithmetic took 19.0 us instead of 16.3 (which has the
+// prefactors of k_step's sTan too).  Zeros are inside because a wall contact's
+// tangential velocity has them (with them outside, one step of 10,000 17.8 us
+// instead of 17.4).
+// blaze_check_division compares it with IEEE division on the GPU.
 __device__ __forceinline__ float div_rn(float a, float y, float b) {
-  if (a == 0.0f) return a * y;
-  if (!(fabsf(a) >= 1e-20f && fabsf(a) <= 1e15f)) return a / b;
   const float q0 = a * y;
   const float q1 = fmaf(fmaf(-q0, b, a), y, q0);
-  const float r1 = fmaf(-q1, b, a);
-  return r1 == 0.0f ? q1 : fmaf(r1, y, q1);
+  return copysignf(fmaf(fmaf(-q1, b, a), y, q1), a);
 }
 __device__ __forceinline__ float3 div3_rn(float3 a, float b) {
-  if (!(b >= 1e-15f && b <= 1e15f)) return f3(a.x / b, a.y / b, a.z / b);
-  const float y = __frcp_rn(b);
-  return f3(div_rn(a.x, y, b), div_rn(a.y, y, b), div_rn(a.z, y, b));
+  const uint32_t x = __float_as_uint(fabsf(a.x)), y = __float_as_uint(fabsf(a.y)),
+                 z = __float_as_uint(fabsf(a.z));
+  const bool in = b >= 1e-15f && b <= 1e15f &&
+                  umin(umin(x - 1u, y - 1u), z - 1u) >= __float_as_uint(1e-20f) - 1u &&
+                  umax(umax(x, y), z) <= __float_as_uint(1e15f);
+  if (!in) return f3(a.x / b, a.y / b, a.z / b);
+  const float r = __frcp_rn(b);
+  return f3(div_rn(a.x, r, b), div_rn(a.y, r, b), div_rn(a.z, r, b));
 }
 
 }  // namespace blaze
