@@ -700,24 +700,45 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     int best = -1;
     float best_d = 0.0f;
     bool face = false;
-    for (uint32_t q = o0; q < o1; ++q) {
-      // most of a cell's triangles are out of reach: a sphere around each
-      // tells (rounded up by more than the test's own rounding, tri_bound)
-      const float4 bs = __ldg(g.stri_b + q);
-      const float3 dc = pd - xyz(bs);
-      const float reach = bs.w + ra;
-      if (dot3(dc, dc) > reach * reach) continue;
-      const int id = (int)__ldg(g.stri_ids + q);
-      float3 nrm;
-      float delta;
-      int region;
-      if (!wall_touch<kCurved>(g.walls[id], pd, ra, nrm, delta, region)) continue;
-      if (region == 0) {
-        face = true;
-        if (q - o0 < 32u) keep |= 1u << (q - o0);
-      } else if (best < 0 || delta > best_d) {
-        best = (int)(q - o0);
-        best_d = delta;
+    // A particle's candidates are tested by the whole warp, one per lane: few of
+    // a warp's particles are near the mesh, and with each tested by its own lane
+    // the others wait for a chain of dependent loads: mixed charge of 21,000, 32
+    // steps, 1.41 -> 1.25-1.30 ms (alone 3.04 -> 2.66); 100,000 spheres in a drum
+    // of 16,384 triangles 23.0 -> 19.3 us a step.
+    for (unsigned near = __ballot_sync(kAll, o1 > o0); near; near &= near - 1u) {
+      const int src = __ffs(near) - 1;
+      const uint32_t c0 = __shfl_sync(kAll, o0, src), c1 = __shfl_sync(kAll, o1, src);
+      const float rp = __shfl_sync(kAll, ra, src);
+      const float3 pp = f3(__shfl_sync(kAll, pd.x, src), __shfl_sync(kAll, pd.y, src),
+                           __shfl_sync(kAll, pd.z, src));
+      for (uint32_t q0 = c0; q0 < c1; q0 += 32u) {
+        const uint32_t q = q0 + (uint32_t)lane;
+        bool hit = false;
+        int region = 0;
+        float delta = 0.0f;
+        if (q < c1) {
+          // most of a cell's triangles are out of reach: a sphere around each
+          // tells (rounded up by more than the test's own rounding, tri_bound)
+          const float4 bs = __ldg(g.stri_b + q);
+          const float3 dc = pp - xyz(bs);
+          const float reach = bs.w + rp;
+          float3 nrm;
+          if (!(dot3(dc, dc) > reach * reach))
+            hit = wall_touch<kCurved>(g.walls[__ldg(g.stri_ids + q)], pp, rp, nrm, delta, region);
+        }
+        const unsigned on_face = __ballot_sync(kAll, hit && region == 0);
+        // overlaps are positive: their bits sort as they do; the first of equals
+        const uint32_t depth = hit && region != 0 ? __float_as_uint(delta) : 0u;
+        const uint32_t most = __reduce_max_sync(kAll, depth);
+        const int first = __ffs(__ballot_sync(kAll, depth == most)) - 1;
+        if (lane == src) {
+          if (on_face) face = true;
+          if (q0 == c0) keep = on_face;
+          if (most && (best < 0 || __uint_as_float(most) > best_d)) {
+            best = (int)(q0 - c0) + first;
+            best_d = __uint_as_float(most);
+          }
+        }
       }
     }
     // the lanes' next kept candidates, ascending: of the first 32 by the mask,
