@@ -593,7 +593,7 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
   }
   __syncthreads();
   const SimParams& P = *Pg;
-  // The tangential factor of a contact (two divisions) depends on the two types
+  // The tangential factor of a contact (it has a division) depends on the two types
   // only: a table per block where a lane walks its own contacts.  A step whose
   // contacts are few and shared by a warp does not win back the table's wait
   // (one step of 10,000: 18.0 us with it, 17.8 without).
