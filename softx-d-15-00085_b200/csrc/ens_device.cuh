@@ -154,6 +154,13 @@ __device__ __forceinline__ float3 closest_on_triangle(float3 p, float3 a, float3
   return a + ab * (vb * den) + ac * (vc * den);
 }
 
+// Whether a sphere at p may touch plane W: an FP32 test whose margin is ten
+// times the FP32 rounding of the distance.
+__device__ __forceinline__ bool plane_near(const EnsWallDev& W, float3 p, float r) {
+  const float mag = fabsf(p.x) + fabsf(p.y) + fabsf(p.z) + fabsf(W.r);
+  return dot3(W.a, p) - W.r < r + 1e-6f * mag;
+}
+
 // Contact of a sphere (centre p, radius r) with one wall: normal from the
 // wall to the centre, overlap; false when not touching.  kCurved = false
 // compiles the plane test only (ensembles whose walls are all planes).
@@ -163,9 +170,8 @@ __device__ __forceinline__ bool wall_touch(const EnsWallDev& W, float3 p, float 
   region = 0;
   // Walls first take a conservative FP32 test (its margin is ten times the
   // FP32 rounding of the distance), so the FP64 overlap runs only near them.
-  const float mag = fabsf(p.x) + fabsf(p.y) + fabsf(p.z) + fabsf(W.r);
   if (W.kind == kWallPlane) {
-    if (!(dot3(W.a, p) - W.r < r + 1e-6f * mag)) return false;
+    if (!plane_near(W, p, r)) return false;
     delta = overlap_plane(r, W.a, W.r, p);
     if (!(delta > 0.0f)) return false;
     n = W.a;
@@ -174,6 +180,7 @@ __device__ __forceinline__ bool wall_touch(const EnsWallDev& W, float3 p, float 
   if constexpr (!kCurved) return false;
   if (W.kind == kWallCylinder) {
     {
+      const float mag = fabsf(p.x) + fabsf(p.y) + fabsf(p.z) + fabsf(W.r);
       const float3 v = p - W.a;
       if (!(len3(v - dot3(v, W.b) * W.b) + r > W.r - 1e-6f * (mag + 2.0f * W.r))) return false;
     }

@@ -668,19 +668,44 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     }
     held += __popc(bal);
   };
+  // Planes only: most warps are near no wall, so every lane first takes its
+  // walls' conservative test alone, and only walls that some lane is near are
+  // met by the warp.  With the vote and the full test at every wall a loose bed
+  // of 400,000 took 17.3 us a step instead of 15.2, one of 2,000,000 74 instead
+  // of 67, and 512 beds of 7.4 million settling from rest 343 instead of 259.
+  // With a mesh, where most walls are triangles (below), it costs more than it
+  // gives: hopper of 400,000, 82 against 79 us.
   const int nwall = valid ? S.nwall : 0;
   const int nwall_most = __reduce_max_sync(kAll, nwall);
-  for (int w = 0; w < nwall_most; ++w) {
-    float3 nrm = f3(0.0f, 0.0f, 0.0f);
-    float delta = 0.0f;
-    int region;
-    bool hit = false, moving = false;
-    if (w < nwall) {
-      const EnsWallDev& W = g.walls[S.wall0 + w];
-      hit = wall_touch<kCurved>(W, pa, ra, nrm, delta, region);
-      moving = rot && W.turning;
+  if constexpr (kCurved) {
+    for (int w = 0; w < nwall_most; ++w) {
+      float3 nrm = f3(0.0f, 0.0f, 0.0f);
+      float delta = 0.0f;
+      int region;
+      bool hit = false, moving = false;
+      if (w < nwall) {
+        const EnsWallDev& W = g.walls[S.wall0 + w];
+        hit = wall_touch<kCurved>(W, pa, ra, nrm, delta, region);
+        moving = rot && W.turning;
+      }
+      wall_contact(hit, S.wall0 + w, nrm, delta, moving);
     }
-    wall_contact(hit, S.wall0 + w, nrm, delta, moving);
+  } else {
+    for (int w0 = 0; w0 < nwall_most; w0 += 32) {
+      const int first = S.wall0 + w0, wn = min(32, nwall - w0);
+      uint32_t near = 0u;
+      for (int w = 0; w < wn; ++w)
+        if (plane_near(g.walls[first + w], pa, ra)) near |= 1u << w;
+      for (uint32_t any = __reduce_or_sync(kAll, near); any; any &= any - 1u) {
+        const int w = __ffs(any) - 1;
+        float3 nrm = f3(0.0f, 0.0f, 0.0f);
+        float delta = 0.0f;
+        int region;
+        const bool hit = (near >> w & 1u) != 0u &&
+                         wall_touch<kCurved>(g.walls[first + w], pa, ra, nrm, delta, region);
+        wall_contact(hit, first + w, nrm, delta, false);   // only curved builds turn
+      }
+    }
   }
   if (kCurved && g.tri_off) {
     const float3 pd = rot ? S.rot_o + rot_about(S.rot_a, rc, -rsn, pa - S.rot_o) : pa;

@@ -173,3 +173,41 @@ def test_polyhedra_on_a_fine_mesh(side):
     assert (a["vel"][rocks, 2] > 0).any()            # some have bounced
     ens.close()
     o.close()
+
+
+@pytest.mark.parametrize("facets", [26, 28, 29, 70])
+def test_many_planes(facets):
+    """A prism of plane walls around one system (32, 33 and more walls with top,
+    floor and two slanted planes: the walls are tested 32 at a time) and a plain
+    box beside it, so one warp holds particles with different wall counts."""
+    r, n = 0.2, 101
+    pos, rng, side = lattice(n, 0.4 - 2e-4, 0.2, facets)
+    c, L, H = 0.5 * side, side + 0.02, 1.5 * side + 1.0
+    W, R = [], 0.5 * side + 0.01
+    for k in range(facets):
+        a = 2.0 * math.pi * (k + 0.5) / facets
+        m = np.array([-math.cos(a), -math.sin(a), 0.0])
+        W.append(E.plane(m, float(m @ [c, c, 0.0]) - R))
+    W += [E.plane((0, 0, 1), 0.0), E.plane((0, 0, -1), -H)]
+    for s in (1.0, -1.0):
+        m = np.array([s, 0.0, 1.0]) / math.sqrt(2.0)
+        W.append(E.plane(m, float(m @ [c - s * 0.5 * side, c, 0.3])))
+    kw = dict(density=2500e-6, kn=1e5, restitution=0.6, mu=0.4)
+    A = synth.box_system(n, L, H, 0.45, 0, **kw)
+    A.nwalls = len(W)
+    B = synth.box_system(n, L, H, 0.45, len(W), **kw)
+    W += synth.box_walls(L, H)
+    pos = np.concatenate([pos, pos])
+    rad = np.full(2 * n, r, np.float32)
+    vel = rng.normal(scale=60.0, size=pos.shape).astype(np.float32)
+    o = EnsRestated([A, B], W, E.LAW_LINEAR, 5e-6, 0.02, 32, precision="f32")
+    ens = E.Ensemble([A, B], W, law=E.LAW_LINEAR, dt=5e-6, skin=0.02, use_graph=1)
+    for e in (o, ens):
+        e.set_state(pos, rad, vel)
+        e.step(40)
+    a, b = ens.state(), o.state()
+    assert a["status"] == b["status"]
+    for k in ("pos", "vel", "avel"):
+        np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
+    ens.close()
+    o.close()
