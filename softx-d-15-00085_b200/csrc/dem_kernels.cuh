@@ -120,9 +120,9 @@ __device__ __forceinline__ bool list_needs_rebuild(float skin, const StepLink& l
 // contacts among its lanes, so with fewer particles its chain of dependent
 // loads and laws is shorter; where full warps would not fill the GPU (148 SMs
 // of 24 warps) the particles are spread over more of them.
-inline int warp_particles(int n) {
+inline int warp_particles(int n, int warps = 148 * 24) {
   int p = 32;
-  while (p > 4 && (n + p / 2 - 1) / (p / 2) <= 148 * 24) p /= 2;
+  while (p > 4 && (n + p / 2 - 1) / (p / 2) <= warps) p /= 2;
   return p;
 }
 // blocks of `threads` that hold n particles, wp to a warp

@@ -1012,9 +1012,16 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int nbl
   return s_ok != 0;
 }
 
-// Registers capped at the step kernel's count, so as many blocks stay
-// resident as the per-step launches have.
-constexpr int kPersistRegs = kStepRegs;
+// Registers as the small step's: kEnsOneWave particles are one per resident
+// lane.  A box of 113,000 settling from rest at 64 and 80: 11.0 and 9.8 us a step.
+constexpr int kPersistRegs = kStepRegsSmall;
+// Particles per warp of the persistent step: spread over at most a third of the
+// resident warps.  A grid that fills the GPU makes ensembles stepped side by
+// side wait for one another: three boxes of 16,000 at 4, 16 and 32 per warp
+// 11.8, 6.2 and 6.4 us a step.
+inline int persist_warp_particles(int law, int n) {
+  return law == kLawReference ? 32 : warp_particles(n, kEnsOneWave / 32 / 3);
+}
 
 // Self-check of the barrier's bounded wait: the barrier is told of one
 // block more than the launch has, so nothing completes it; every block must
@@ -1235,7 +1242,7 @@ int ens_persist_grid(const EnsGeom& g, int block, int n) {
               ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_persist<kLawHertz, false>, block, contact_bytes(block))
               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_persist<kLawLinear, false>, block, contact_bytes(block));
   if (err != cudaSuccess || per_sm < 1) return 0;
-  const int need = warp_blocks(n, ens_warp_particles(g.law, n), block);
+  const int need = warp_blocks(n, persist_warp_particles(g.law, n), block);
   return std::max(1, std::min(need, per_sm * sms));
 }
 
@@ -1253,16 +1260,17 @@ cudaError_t ens_launch_persist(const EnsGeom& g, const EnsBufs& b, int home, int
   cfg.attrs = attr;
   cfg.numAttrs = coop ? 1 : 0;
   const StateBuf sh = b.S[home], so = b.S[home ^ 1], ss = b.S[2];
+  const int wp = persist_warp_particles(g.law, n);
   if (g.law == kLawReference)
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawReference, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawReference, false>, g, b, sh, so, ss, n, wp, ctl, rebuilt, p);
   if (g.curved) {
     if (g.law == kLawHertz)
-      return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, true>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, true>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
+      return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, true>, g, b, sh, so, ss, n, wp, ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, true>, g, b, sh, so, ss, n, wp, ctl, rebuilt, p);
   }
   if (g.law == kLawHertz)
-    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
-  return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, false>, g, b, sh, so, ss, n, ens_warp_particles(g.law, n), ctl, rebuilt, p);
+    return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawHertz, false>, g, b, sh, so, ss, n, wp, ctl, rebuilt, p);
+  return cudaLaunchKernelEx(&cfg, k_ens_persist<kLawLinear, false>, g, b, sh, so, ss, n, wp, ctl, rebuilt, p);
 }
 
 void ens_launch_rot_tick(const EnsGeom& g, int nsys, const RoundLink& round, cudaStream_t st) {

@@ -307,8 +307,8 @@ void ens_launch_nlist(const EnsGeom& g, const EnsBufs& b, int n, const CellSort&
 // Particles per warp (warp_particles); the reference law walks a particle's
 // contacts on its own lane.
 inline int ens_warp_particles(int law, int n) { return law == kLawReference ? 32 : warp_particles(n); }
-// particles that the step's resident grid holds, a lane each (148 SMs, three
-// blocks of 256)
+// particles that the resident grid of a kernel at 80 registers holds, a lane
+// each (148 SMs, three blocks of 256)
 constexpr int kEnsOneWave = 148 * 3 * 256;
 // `block`: threads per block (64 .. kMaxStepBlock, a multiple of 32).
 constexpr int kMaxStepBlock = 512;
