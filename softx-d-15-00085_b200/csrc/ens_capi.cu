@@ -52,6 +52,7 @@ struct blaze_ens {
   uint32_t* d_tri_ids = nullptr;
   float4* d_tri_b = nullptr;
   bool curved = false;        // some wall is a cylinder or a triangle
+  EnsLaunch forced{};         // blaze_ens_set_launch: 0 by size (resident: -1 / 1)
   uint32_t ncell_tab = 0;
   EnsBufs b{};
   int cur = 0;
@@ -146,6 +147,12 @@ EnsGeom geom(const blaze_ens* e) {
     g.mix.st = e->d_pst;
     g.mix.npoly = e->npoly;
   }
+  const EnsLaunch& f = e->forced;
+  g.launch.warp_particles = f.warp_particles && e->opt.law != kLawReference
+                                ? f.warp_particles
+                                : ens_warp_particles(e->opt.law, e->n);
+  g.launch.resident = f.resident ? f.resident > 0 : e->n <= kEnsOneWave;
+  g.launch.poly_warps = f.poly_warps ? f.poly_warps : mix_warps(e->npoly);
   return g;
 }
 
@@ -1112,6 +1119,18 @@ int blaze_ens_step(blaze_ens* e, int nsteps) {
   e->last_launches = 0;
   if (nsteps > 0) e->stepped = true;
   return advance(e, nsteps, e->opt.use_graph != 0 && !e->prof);
+}
+
+int blaze_ens_set_launch(blaze_ens* e, int warp_particles, int registers, int poly_warps) {
+  if (!e || (warp_particles != 0 && warp_particles != 4 && warp_particles != 8 &&
+             warp_particles != 16 && warp_particles != 32) ||
+      (registers != 0 && registers != 64 && registers != 80) ||
+      (poly_warps != 0 && poly_warps != 1 && poly_warps != 2 && poly_warps != 4))
+    return -1;
+  CK(cudaStreamSynchronize(e->stream));
+  e->forced = EnsLaunch{warp_particles, registers == 0 ? 0 : (registers == 80 ? 1 : -1), poly_warps};
+  drop_graphs(e);
+  return 0;
 }
 
 int blaze_ens_set_profile(blaze_ens* e, int on) {

@@ -1158,12 +1158,12 @@ void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl
                      StepLink link, const EnsCapture* cap, int block, cudaStream_t st) {
   const EnsCapture c = cap ? *cap : EnsCapture{nullptr, nullptr};
   const int bs = block >= 64 && block <= kMaxStepBlock && block % 32 == 0 ? block : kThreads;
-  const int wp = ens_warp_particles(g.law, n);
+  const int wp = g.launch.warp_particles;
   const int gs = warp_blocks(n, wp, bs);
 #define ENS_ARGS g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, wp, ctl, link, c
 #define ENS_LAUNCH(...)                                                             \
   do {                                                                              \
-    if (n <= kEnsOneWave)                                                              \
+    if (g.launch.resident)                                                          \
       k_ens_step<__VA_ARGS__, true><<<gs, bs, contact_bytes(bs), st>>>(ENS_ARGS);   \
     else                                                                            \
       k_ens_step<__VA_ARGS__, false><<<gs, bs, contact_bytes(bs), st>>>(ENS_ARGS);  \
@@ -1220,7 +1220,7 @@ void ens_launch_step(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl
 void ens_launch_step_record(const EnsGeom& g, const EnsBufs& b, int cur, int n, StepCtl* ctl,
                             StepLink link, const EnsTape& tape, int block, cudaStream_t st) {
   const int bs = block >= 64 && block <= kMaxStepBlock && block % 32 == 0 ? block : kThreads;
-  const int wp = ens_warp_particles(g.law, n);
+  const int wp = g.launch.warp_particles;
   const int gs = warp_blocks(n, wp, bs);
   // reverse mode accepts plane walls only (blaze_ens_adj_create)
   k_ens_step_rec<<<gs, bs, contact_bytes(bs), st>>>(g, b, b.S[cur], b.S[2], b.S[cur ^ 1], n, wp, ctl, link, tape);

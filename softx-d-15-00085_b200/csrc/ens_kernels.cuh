@@ -148,6 +148,14 @@ struct MixView {
   int npoly;                 // 0: spheres only
 };
 
+// The shapes of a step's launches, by size unless a test asks for others
+// (blaze_ens_set_launch).
+struct EnsLaunch {
+  int warp_particles;   // particles per warp of the sphere step (ens_warp_particles)
+  int resident;         // 1: its build for grids that the GPU holds at once (kEnsOneWave)
+  int poly_warps;       // warps per polyhedron (mix_warps)
+};
+
 struct EnsGeom {
   const EnsSysDev* sys;
   const EnsWallDev* walls;
@@ -164,6 +172,7 @@ struct EnsGeom {
   float2* rot;               // per system: (cos, sin) of the drum's turn so far
   int any_rot;               // 1: some system turns (the step compiled with the turn)
   MixView mix;
+  EnsLaunch launch;          // (host)
 };
 
 struct EnsCapture { float4* f; float4* t; };

@@ -7,8 +7,6 @@ namespace blaze {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kMixWarps = 4;      // warps per polyhedron in the step
-constexpr int kMixBlock = 32 * kMixWarps;
 constexpr int kMixHits = 32;      // touching triangles kept per polyhedron and step
 
 inline int nblk(int n) { return (n + kThreads - 1) / kThreads; }
@@ -338,6 +336,7 @@ __device__ bool hull_tri_warp(int lane, const HullRef& D, const double3* T, doub
                          kind);
 }
 
+template <int kWarps>
 struct MixSmem {
   float4 f[kMixSlots];      // per slot: force and torque on this polyhedron
   float4 t[kMixSlots];
@@ -345,13 +344,13 @@ struct MixSmem {
   double4 fn[kMixMaxF];
   uint32_t polys[2];        // slots whose polyhedron's bounding sphere overlaps
   uint32_t touch[2];        // slots in contact
-  uint32_t nearby[kMixWarps];  // of a window of kMixBlock candidate triangles
+  uint32_t nearby[kWarps];  // of a window of 32 kWarps candidate triangles
   int task;                 // next task of the window
   // the window's nearby triangles, in ascending order
-  double3 nd[kMixBlock];    // unrounded normal
-  MixHit hit[kMixBlock];
-  int id[kMixBlock];
-  int kind[kMixBlock];      // 0: the triangle's face; 1, 2: a face of the polyhedron, an edge
+  double3 nd[32 * kWarps];  // unrounded normal
+  MixHit hit[32 * kWarps];
+  int id[32 * kWarps];
+  int kind[32 * kWarps];    // 0: the triangle's face; 1, 2: a face of the polyhedron, an edge
                             // pair; -1: apart
   // the touching triangles
   double3 knd[kMixHits];
@@ -371,22 +370,22 @@ __device__ __forceinline__ float3 mat_tvec_f(const float* R, float3 v) {
             (R[2] * v.x + R[5] * v.y) + R[8] * v.z);
 }
 
-// A block of kMixWarps warps per polyhedron.  A polyhedron is a long chain of
-// tests (the spheres around it, the polyhedra around it one at a time, the
-// triangles near it one at a time), and a charge has few of them: with a warp
+// A block of kWarps warps per polyhedron (mix_warps).  A polyhedron is a long
+// chain of tests (the spheres around it, the polyhedra around it one at a time,
+// the triangles near it one at a time), and a charge has few of them: with a warp
 // each, 1,000 rocks filled 8 % of the warp slots and the step took as long as
 // the rock with the most neighbours and triangles.  Here the tests are tasks
-// that the block's warps take in turn (1,000 rocks among 20,000 balls in the
-// turning drum, 32 steps: 1.49 -> 1.37 ms, one state alone 3.58 -> 3.15).  Every test is
+// that the block's warps take in turn.  Every test is
 // evaluated as one warp did, and the results are summed in the same order:
 // the polyhedron's own force by one lane in slot order, then the walls
 // (planes in order, then the kept triangles in ascending id), as the
 // restatement sums.
-template <bool kCapture, bool kRot>
-__global__ void __launch_bounds__(kMixBlock, 4)
+template <int kWarps, bool kCapture, bool kRot>
+__global__ void __launch_bounds__(32 * kWarps, 16 / kWarps)
 k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_sorted,
                 StateBuf out, StepCtl* ctl, StepLink link, EnsCapture cap) {
-  __shared__ MixSmem sm;
+  constexpr int kBlock = 32 * kWarps;
+  __shared__ MixSmem<kWarps> sm;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int p = blockIdx.x;
   if (!round_runs(link.round)) return;
@@ -416,11 +415,10 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
   const uint32_t mlo = L.mlo[p], mhi = L.mhi[p];
   uint32_t st = 0;
 
-  // the polyhedra whose bounding spheres overlap this one's (two warps, a
-  // slot per lane)
-  if (threadIdx.x < 2) sm.touch[threadIdx.x] = 0u;
-  if (wid < 2) {
-    const uint32_t k = (uint32_t)threadIdx.x;
+  // the polyhedra whose bounding spheres overlap this one's (a slot per lane,
+  // a warp per 32 slots)
+  for (int half = wid; half < 2; half += kWarps) {
+    const uint32_t k = (uint32_t)(lane + 32 * half);
     bool pair = false;
     if (k < cnt) {
       const float4 pb4 = in.pos[L.idx[(size_t)k * P + p]];
@@ -431,7 +429,10 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
       }
     }
     const uint32_t bal = __ballot_sync(0xffffffffu, pair);
-    if (lane == 0) sm.polys[wid] = bal;
+    if (lane == 0) {
+      sm.polys[half] = bal;
+      sm.touch[half] = 0u;
+    }
   }
 
   // a sphere neighbour per lane, slots 32 half + lane
@@ -548,7 +549,7 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
   if (o1 > o0 && rot) {
     const double3 ax = d3(S.rot_a);
     const double cc = (double)rc, ss = -(double)rsn;
-    for (int it = (int)threadIdx.x; it < A.nv + A.nf; it += kMixBlock) {
+    for (int it = (int)threadIdx.x; it < A.nv + A.nf; it += kBlock) {
       if (it < A.nv) {
         const double3 v = rot_about_d(ax, cc, ss, dxyz(A.V[it]));
         sm.v[it] = make_double4(v.x, v.y, v.z, 0.0);
@@ -561,11 +562,11 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
     D.V = sm.v;
     D.F = sm.fn;
   }
-  // Windows of kMixBlock candidate triangles; the first window's tasks are
+  // Windows of kBlock candidate triangles; the first window's tasks are
   // also the spheres and the polyhedra.
   const float lim = rb * 1.001f + 1e-3f;
   bool first = true;
-  for (uint32_t q0 = o0; first || q0 < o1; q0 += kMixBlock, first = false) {
+  for (uint32_t q0 = o0; first || q0 < o1; q0 += kBlock, first = false) {
     const uint32_t qq = q0 + threadIdx.x;
     bool near = false;
     int id = -1;
@@ -588,7 +589,7 @@ k_mix_poly_step(EnsGeom g, EnsBufs b, MixBufs m, StateBuf in_plain, StateBuf in_
     __syncthreads();
     int at = 0, nnear = 0;
 #pragma unroll
-    for (int w = 0; w < kMixWarps; ++w) {
+    for (int w = 0; w < kWarps; ++w) {
       if (w < wid) at += __popc(sm.nearby[w]);
       nnear += __popc(sm.nearby[w]);
     }
@@ -840,15 +841,23 @@ void mix_launch_poly_step(const EnsGeom& g, const EnsBufs& b, const MixBufs& m, 
                           StepCtl* ctl, StepLink link, const EnsCapture* cap, cudaStream_t st) {
   if (m.npoly <= 0) return;
   const EnsCapture c = cap ? *cap : EnsCapture{nullptr, nullptr};
-  const int gs = m.npoly;
 #define MIX_ARGS g, b, m, b.S[cur], b.S[2], b.S[cur ^ 1], ctl, link, c
+#define MIX_STEP(W, C, R) k_mix_poly_step<W, C, R><<<m.npoly, 32 * W, 0, st>>>(MIX_ARGS)
+#define MIX_STEP_W(C, R)                                \
+  do {                                                  \
+    if (g.launch.poly_warps == 4) MIX_STEP(4, C, R);    \
+    else if (g.launch.poly_warps == 2) MIX_STEP(2, C, R); \
+    else MIX_STEP(1, C, R);                             \
+  } while (0)
   if (g.any_rot) {
-    if (cap) k_mix_poly_step<true, true><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
-    else k_mix_poly_step<false, true><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
+    if (cap) MIX_STEP_W(true, true);
+    else MIX_STEP_W(false, true);
   } else {
-    if (cap) k_mix_poly_step<true, false><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
-    else k_mix_poly_step<false, false><<<gs, kMixBlock, 0, st>>>(MIX_ARGS);
+    if (cap) MIX_STEP_W(true, false);
+    else MIX_STEP_W(false, false);
   }
+#undef MIX_STEP_W
+#undef MIX_STEP
 #undef MIX_ARGS
 }
 

@@ -211,3 +211,36 @@ def test_many_planes(facets):
         np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
     ens.close()
     o.close()
+
+
+@pytest.mark.parametrize("warps", [1, 2, 4])
+def test_warps_per_polyhedron(warps):
+    """A rock's tests by one warp, or by two or four in turn: rocks and balls poured on
+    each other, and thrown on a floor of more than a window of triangles."""
+    L, H = 8.0, 14.0
+    S, W, p, r, sh, so, q = synth.mixed_box_ensemble(n_spheres=60, n_rocks=14, L=L, H=H, kn=1e5)
+    x = np.linspace(0.0, L, 17)
+    W = [w for k, w in enumerate(W) if k != 4]
+    for i in range(16):
+        for j in range(16):
+            a, b = (x[i], x[j], 0.0), (x[i + 1], x[j], 0.0)
+            c, d = (x[i + 1], x[j + 1], 0.0), (x[i], x[j + 1], 0.0)
+            W += [E.triangle(a, b, c), E.triangle(a, c, d)]
+    s = S[0]
+    s.nwalls, s.tri0, s.ntris = 5, 5, len(W) - 5
+    vel = np.zeros_like(p)
+    vel[:, 2] = -60.0 - 6.0 * p[:, 2]                # the upper ones catch up
+    ens = E.Ensemble(S, W, law=E.LAW_LINEAR, dt=1e-5, skin=0.04, use_graph=1)
+    ens.set_launch(poly_warps=warps)
+    o = EnsRestated(S, W, E.LAW_LINEAR, 1e-5, 0.04, 32, precision="f32")
+    for e in (ens, o):
+        e.set_state(p, r, vel)
+        e.set_polyhedra(sh, so, q)
+        e.step(1600)
+    a, b = ens.state(), o.state()
+    assert a["status"] == b["status"] == 0
+    for k in ("pos", "vel", "avel"):
+        np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
+    np.testing.assert_array_equal(ens.orientations().astype(np.float64), o.orientations())
+    ens.close()
+    o.close()
