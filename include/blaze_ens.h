@@ -144,12 +144,14 @@ int blaze_ens_rebuild_kernels(blaze_ens* e);
  * zero-work launches when no re-sort is due), the polyhedron geometry, the
  * polyhedron step, the sphere step.  Turning it on clears the sums. */
 int blaze_ens_set_profile(blaze_ens* e, int on);
-/* The launch shapes of the steps, which the sizes choose otherwise (0): the
- * particles that a warp takes (4, 8, 16 or 32; the reference law always 32),
+/* The launch shapes of the steps, which the sizes choose otherwise (0): graph
+ * stepping in rounds of steps (1) or with a conditional node before every step
+ * (-1), the particles that a warp takes (4, 8, 16 or 32; the reference law always 32),
  * the step kernel's registers (64 or 80), the warps that take a polyhedron
  * (1, 2 or 4).  For tests and measurements: the results are the same bits.  Not
  * for the persistent kernel. */
-int blaze_ens_set_launch(blaze_ens* e, int warp_particles, int registers, int poly_warps);
+int blaze_ens_set_launch(blaze_ens* e, int rounds, int warp_particles, int registers,
+                         int poly_warps);
 /* ms4: the four sums in ms; steps: the plain steps they cover. */
 int blaze_ens_profile(blaze_ens* e, float* ms4, int* steps);
 

@@ -269,10 +269,11 @@ class Ensemble:
     def rebuild_kernels(self):
         return self.lib.blaze_ens_rebuild_kernels(self.h)
 
-    def set_launch(self, warp_particles=0, registers=0, poly_warps=0):
+    def set_launch(self, rounds=0, warp_particles=0, registers=0, poly_warps=0):
         """Launch shapes of the steps (blaze_ens_set_launch); 0: by size."""
-        _check(self.lib.blaze_ens_set_launch(self.h, C.c_int(warp_particles), C.c_int(registers),
-                                             C.c_int(poly_warps)), "blaze_ens_set_launch")
+        _check(self.lib.blaze_ens_set_launch(self.h, C.c_int(rounds), C.c_int(warp_particles),
+                                             C.c_int(registers), C.c_int(poly_warps)),
+               "blaze_ens_set_launch")
 
     def set_profile(self, on):
         _check(self.lib.blaze_ens_set_profile(self.h, int(bool(on))), "blaze_ens_set_profile")

@@ -53,6 +53,7 @@ struct blaze_ens {
   float4* d_tri_b = nullptr;
   bool curved = false;        // some wall is a cylinder or a triangle
   EnsLaunch forced{};         // blaze_ens_set_launch: 0 by size (resident: -1 / 1)
+  int rounds = 0;             // the same: -1 never, 1 always
   uint32_t ncell_tab = 0;
   EnsBufs b{};
   int cur = 0;
@@ -73,7 +74,7 @@ struct blaze_ens {
   cudaGraphExec_t graph[2] = {nullptr, nullptr};    // steps from S[c] (build_round_graph, build_if_graph)
   cudaGraphExec_t pgraph[2] = {nullptr, nullptr};   // persistent stepping, home S[c]
   int* d_pw = nullptr;        // persistent stepping: left, done, req_step, barrier x3; from 8 on
-                              // the rounds of graph stepping: left, stop, at, want
+                              // the rounds of graph stepping (EnsRound)
   float2* d_rot = nullptr;    // per system: (cos, sin) of the drum's turn so far
   bool any_rot = false;
   int persist_grid = 0;
@@ -509,13 +510,14 @@ int enqueue_step(blaze_ens* e) {
 }
 
 EnsRound round_words(const blaze_ens* e) {
-  return EnsRound{e->d_pw + 8, e->d_pw + 9, e->d_pw + 10, e->d_pw + 11};
+  int* w = e->d_pw + 8;
+  return EnsRound{w, w + 1, w + 2, w + 3, w + 4, w + 5, w + 6};
 }
 
-// The conditional node (IF or WHILE) on h added to the graph being captured
-// on cs; its body in *body.
+// The conditional node (IF, WHILE or SWITCH) on h added to the graph being
+// captured on cs; its nbody bodies in bodies[].
 int add_conditional(cudaStream_t cs, cudaGraphConditionalHandle h,
-                    cudaGraphConditionalNodeType type, cudaGraph_t* body) {
+                    cudaGraphConditionalNodeType type, cudaGraph_t* bodies, int nbody = 1) {
   cudaStreamCaptureStatus status;
   cudaGraph_t capg = nullptr;
   const cudaGraphNode_t* deps = nullptr;
@@ -527,10 +529,10 @@ int add_conditional(cudaStream_t cs, cudaGraphConditionalHandle h,
   cp.type = cudaGraphNodeTypeConditional;
   cp.conditional.handle = h;
   cp.conditional.type = type;
-  cp.conditional.size = 1;
+  cp.conditional.size = (unsigned)nbody;
   cudaGraphNode_t node;
   CK(cudaGraphAddNode(&node, capg, deps, ndeps, &cp));
-  *body = cp.conditional.phGraph_out[0];
+  for (int k = 0; k < nbody; ++k) bodies[k] = cp.conditional.phGraph_out[k];
   CK(cudaStreamUpdateCaptureDependencies(cs, &node, 1, cudaStreamSetCaptureDependencies));
   return 0;
 }
@@ -574,23 +576,39 @@ int build_if_graph(blaze_ens* e, int c) {
   return 0;
 }
 
-// Small ensembles (kRoundMax particles at most), from S[c]: one graph whose
-// WHILE node runs rounds until the call's steps are done
-// (ens_launch_round_init before each launch).  A round is a gate kernel, an IF
-// node with the re-sort when the round before asked for one, and kRoundSteps
-// steps in a row, of which those behind a step that asks for a re-sort do
-// nothing.  An IF node before every step costs about as much as a small step:
-// a box of 6,000 spheres, 16 steps, 171 us with IF nodes and a lane per
-// particle, 85 us in rounds with four particles to a warp.  The launches that
-// do nothing and the words that every step reads first cost a large ensemble
-// more than its IF nodes where the GPU has other work beside it: three hoppers
-// of 400,000 at once 2.77 against 2.66 ms a pass (one alone 3.91 against 4.08),
-// three mixed charges of 21,000 1.38 against 1.37.
-constexpr int kRoundSteps = 16;   // even: a whole round ends in the buffer it began in
-#ifndef BLAZE_ROUND_MAX
-#define BLAZE_ROUND_MAX 16384
-#endif
-constexpr int kRoundMax = BLAZE_ROUND_MAX;
+// Ensembles of up to kRoundMax particles, from S[c]: one graph whose WHILE node
+// runs rounds until the call's steps are done (ens_launch_round_init before each
+// launch).  A round is a gate kernel and a SWITCH node on its decision: steps in
+// a row, behind a re-sort when the round before asked for one; the steps behind
+// one that asks for a re-sort do nothing.  A round is kRoundSteps long, or
+// kRoundShort where the step before last also asked for its re-sort within
+// that many steps: hot ensembles would launch more steps that do nothing than
+// steps that run.  An IF node before every step costs 6 us whatever the size;
+// the launches that do nothing, and the words that every step reads first, cost
+// a step more the larger the grid, and most where other work fills the GPU.
+// us a step in rounds and with IF nodes, settling from rest (one alone, calls of
+// 2,000 steps; in brackets three side by side, calls of 32):
+//   box of    6,000    5.7 (5.0)   12.2 (6.8)
+//   box of  113,000    7.8 (8.3)   14.2 (9.6)
+//   box of  400,000   16.3 (18.3)  22.3 (18.0)
+//   box of  800,000   31.4 (35.1)  38.1 (33.0)
+//   box of 1,300,000  49.2 (54.7)  53.9 (49.8)
+// With triangles, cylinders or polyhedra a step is longer and re-sorts more often:
+//   hopper of  50,000  48.9 (28.2)  53.5 (27.3)
+//   hopper of 150,000  85.3 (50.5)  89.5 (49.8)
+//   hopper of 400,000 143.8 (82.1) 146.0 (79.2)
+//   drum mesh, 100,000 12.2         19.3
+// and a box of 20,000 that re-sorts every 1, 2, 5 and 15 steps: 68.9, 35.9, 21.5
+// and 9.8 in rounds, 57.6, 35.0, 22.0 and 15.7 with IF nodes (92.8, 47.3, 21.4
+// and 9.8 without the short rounds).
+constexpr int kRoundSteps = 16;   // both even: a whole round ends in the buffer it began in
+constexpr int kRoundShort = 4;
+constexpr int kRoundMax = 1 << 20;
+constexpr int kRoundMaxCurved = 200000;
+bool in_rounds(const blaze_ens* e) {
+  if (e->rounds) return e->rounds > 0;
+  return e->n <= (e->curved || e->npoly > 0 ? kRoundMaxCurved : kRoundMax);
+}
 int build_round_graph(blaze_ens* e, int c) {
   const int saved = e->cur;
   const EnsRound r = round_words(e);
@@ -600,29 +618,34 @@ int build_round_graph(blaze_ens* e, int c) {
   CK(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
   CK(cudaStreamBeginCaptureToGraph(e->stream, g, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
-  cudaGraph_t body = nullptr, ibody = nullptr, tmp = nullptr;
+  cudaGraph_t body = nullptr, kinds[3] = {nullptr, nullptr, nullptr}, tmp = nullptr;
   int rc = add_conditional(e->stream, hw, cudaGraphCondTypeWhile, &body);
   if (rc) return rc;
-  cudaGraphConditionalHandle hi;
-  CK(cudaGraphConditionalHandleCreate(&hi, body, 0, 0));
+  cudaGraphConditionalHandle hs;
+  CK(cudaGraphConditionalHandleCreate(&hs, body, 0, 0));
   CK(cudaStreamBeginCaptureToGraph(e->aux, body, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
-  ens_launch_round_gate(e->ctl, r, e->d_rb, hi, e->aux);
-  rc = add_conditional(e->aux, hi, cudaGraphCondTypeIf, &ibody);
+  ens_launch_round_gate(e->ctl, r, e->d_rb, kRoundSteps, kRoundShort, hs, e->aux);
+  rc = add_conditional(e->aux, hs, cudaGraphCondTypeSwitch, kinds, 3);
   if (rc) return rc;
-  CK(cudaStreamBeginCaptureToGraph(e->aux2, ibody, nullptr, nullptr, 0,
-                                   cudaStreamCaptureModeThreadLocal));
-  CK(cudaMemsetAsync(e->d_rb, 0x01, sizeof(int), e->aux2));
-  rc = enqueue_rebuild(e, nullptr, e->aux2, r.at);
-  CK(cudaStreamEndCapture(e->aux2, &tmp));
-  if (rc) return rc;
-  for (int k = 0; k < kRoundSteps; ++k) {
-    e->cur = c ^ (k & 1);
-    const RoundLink link{r.left, r.stop, k};
-    launch_step_kernels(e, StepLink{e->d_rb, 0, 0, 0, link}, e->aux);
-    if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, link, e->aux);
+  for (int kind = 0; kind < 3; ++kind) {   // steps; re-sort and steps; re-sort and a few
+    CK(cudaStreamBeginCaptureToGraph(e->aux2, kinds[kind], nullptr, nullptr, 0,
+                                     cudaStreamCaptureModeThreadLocal));
+    e->cur = c;
+    if (kind > 0) {
+      CK(cudaMemsetAsync(e->d_rb, 0x01, sizeof(int), e->aux2));
+      rc = enqueue_rebuild(e, nullptr, e->aux2, r.at);
+      if (rc) return rc;
+    }
+    for (int k = 0; k < (kind == 2 ? kRoundShort : kRoundSteps); ++k) {
+      e->cur = c ^ (k & 1);
+      const RoundLink link{r.left, r.stop, k};
+      launch_step_kernels(e, StepLink{e->d_rb, 0, 0, 0, link}, e->aux2);
+      if (e->any_rot) ens_launch_rot_tick(geom(e), e->nsys, link, e->aux2);
+    }
+    CK(cudaStreamEndCapture(e->aux2, &tmp));
   }
-  ens_launch_round_end(e->ctl, r, kRoundSteps, c, hw, e->aux);
+  ens_launch_round_end(e->ctl, r, c, hw, e->aux);
   CK(cudaStreamEndCapture(e->aux, &tmp));
   ens_launch_round_last(e->b, r, e->n, e->stream);
   cudaGraph_t out = nullptr;
@@ -863,8 +886,8 @@ int create_impl(blaze_ens** out, const blaze_system* systems, int nsys, const bl
   CKF(dalloc(&e->ctl, 1));
   CKF(dalloc(&e->d_rb, kGraphSteps));
   CKF(cudaMemset(e->d_rb, 0, sizeof(int) * kGraphSteps));
-  CKF(dalloc(&e->d_pw, 12));
-  CKF(cudaMemset(e->d_pw, 0, sizeof(int) * 12));
+  CKF(dalloc(&e->d_pw, 16));
+  CKF(cudaMemset(e->d_pw, 0, sizeof(int) * 16));
   CKF(dalloc(&e->d_rot, nsys));
   for (int s = 0; s < nsys; ++s) e->any_rot = e->any_rot || systems[s].rot_omega != 0.0f;
   {
@@ -1061,7 +1084,7 @@ int advance(blaze_ens* e, int nsteps, bool graphs) {
     e->last_launches += 3;   // the budget, then one round's gate and step kernels
     return 0;
   }
-  if (graphs && nsteps >= kGraphSteps && e->n <= kRoundMax) {
+  if (graphs && nsteps >= kGraphSteps && in_rounds(e)) {
     const int c = e->cur;
     if (!e->graph[c]) {
       int rc = build_round_graph(e, c);
@@ -1121,13 +1144,15 @@ int blaze_ens_step(blaze_ens* e, int nsteps) {
   return advance(e, nsteps, e->opt.use_graph != 0 && !e->prof);
 }
 
-int blaze_ens_set_launch(blaze_ens* e, int warp_particles, int registers, int poly_warps) {
-  if (!e || (warp_particles != 0 && warp_particles != 4 && warp_particles != 8 &&
+int blaze_ens_set_launch(blaze_ens* e, int rounds, int warp_particles, int registers,
+                         int poly_warps) {
+  if (!e || rounds < -1 || rounds > 1 || (warp_particles != 0 && warp_particles != 4 && warp_particles != 8 &&
              warp_particles != 16 && warp_particles != 32) ||
       (registers != 0 && registers != 64 && registers != 80) ||
       (poly_warps != 0 && poly_warps != 1 && poly_warps != 2 && poly_warps != 4))
     return -1;
   CK(cudaStreamSynchronize(e->stream));
+  e->rounds = rounds;
   e->forced = EnsLaunch{warp_particles, registers == 0 ? 0 : (registers == 80 ? 1 : -1), poly_warps};
   drop_graphs(e);
   return 0;

@@ -921,21 +921,28 @@ __global__ void k_round_init(EnsRound r, int steps, int at) {
   *r.want = at ^ (steps & 1);
 }
 
-__global__ void k_round_gate(StepCtl* ctl, EnsRound r, int* rb, cudaGraphConditionalHandle if_h) {
+__global__ void k_round_gate(StepCtl* ctl, EnsRound r, int* rb, int steps, int few,
+                             cudaGraphConditionalHandle switch_h) {
   const int req = ctl->rebuild_req;
   ctl->rebuild_req = 0;
   *rb = 0;
   *r.stop = 0x7fffffff;
-  cudaGraphSetConditional(if_h, req ? 1u : 0u);
+  const bool hot = req && *r.last > 0 && *r.last <= few;
+  *r.len = hot ? few : steps;
+  if (req) *r.since = 0;
+  cudaGraphSetConditional(switch_h, req ? (hot ? 2u : 1u) : 0u);
 }
 
-__global__ void k_round_end(StepCtl* ctl, EnsRound r, int steps, int home,
+__global__ void k_round_end(StepCtl* ctl, EnsRound r, int home,
                             cudaGraphConditionalHandle loop_h) {
-  int ran = min(steps, *r.left);
-  if (*r.stop < ran) {
+  int ran = min(*r.len, *r.left);
+  const bool stopped = *r.stop < ran;
+  if (stopped) {
     ran = *r.stop + 1;
     ctl->rebuild_req = 1;
   }
+  *r.since += ran;
+  if (stopped) *r.last = *r.since;
   const int left = *r.left - ran;
   *r.left = left;
   *r.at = home ^ (ran & 1);
@@ -1281,14 +1288,14 @@ void ens_launch_round_init(const EnsRound& r, int steps, int at, cudaStream_t st
   k_round_init<<<1, 1, 0, st>>>(r, steps, at);
 }
 
-void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb,
-                           cudaGraphConditionalHandle if_h, cudaStream_t st) {
-  k_round_gate<<<1, 1, 0, st>>>(ctl, r, rb, if_h);
+void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb, int steps, int few,
+                           cudaGraphConditionalHandle switch_h, cudaStream_t st) {
+  k_round_gate<<<1, 1, 0, st>>>(ctl, r, rb, steps, few, switch_h);
 }
 
-void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int steps, int home,
+void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int home,
                           cudaGraphConditionalHandle loop_h, cudaStream_t st) {
-  k_round_end<<<1, 1, 0, st>>>(ctl, r, steps, home, loop_h);
+  k_round_end<<<1, 1, 0, st>>>(ctl, r, home, loop_h);
 }
 
 void ens_launch_round_last(const EnsBufs& b, const EnsRound& r, int n, cudaStream_t st) {

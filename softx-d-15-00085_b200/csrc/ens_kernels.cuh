@@ -332,18 +332,27 @@ void ens_launch_step_record(const EnsGeom& g, const EnsBufs& b, int cur, int n, 
 void ens_launch_rot_tick(const EnsGeom& g, int nsys, const RoundLink& round, cudaStream_t st);
 // Rounds of steps (RoundLink).  Before a call's first round (init): its steps
 // and the buffer S[at] it starts from.  At a round's start (gate): the pending
-// re-sort request into the IF node, *rb = 0.  Every round's steps are launched
+// re-sort request and the round's length into the SWITCH node (0 steps; 1 a re-sort,
+// then the steps; 2 a re-sort, then few), *rb = 0.  Every round's steps are launched
 // as if its state were in S[home] (a re-sort's copy is read instead by the
 // first); a round that runs to its end leaves it there, and one that stops
 // early is followed by a re-sort, which reads S[*r.at].  At its end: the steps
 // it ran off *left, loop_h (the WHILE node around the rounds) set while some
 // are left.  After the last (last): the state copied to S[*r.want], where the
 // host expects it after an even or odd number of steps, if it is not there.
-struct EnsRound { int* left; int* stop; int* at; int* want; };
+struct EnsRound {
+  int* left;    // steps of the call still to run
+  int* stop;    // RoundLink::stop
+  int* at;      // the buffer that holds the state
+  int* want;    // the one it belongs in after the call
+  int* len;     // the round's steps
+  int* since;   // steps since the last re-sort
+  int* last;    // steps from the re-sort before to the one asked for last
+};
 void ens_launch_round_init(const EnsRound& r, int steps, int at, cudaStream_t st);
-void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb,
-                           cudaGraphConditionalHandle if_h, cudaStream_t st);
-void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int steps, int home,
+void ens_launch_round_gate(StepCtl* ctl, const EnsRound& r, int* rb, int steps, int few,
+                           cudaGraphConditionalHandle switch_h, cudaStream_t st);
+void ens_launch_round_end(StepCtl* ctl, const EnsRound& r, int home,
                           cudaGraphConditionalHandle loop_h, cudaStream_t st);
 void ens_launch_round_last(const EnsBufs& b, const EnsRound& r, int n, cudaStream_t st);
 // Persistent stepping: one cooperative launch runs up to *left steps with a

@@ -244,3 +244,52 @@ def test_warps_per_polyhedron(warps):
     np.testing.assert_array_equal(ens.orientations().astype(np.float64), o.orientations())
     ens.close()
     o.close()
+
+
+@pytest.mark.parametrize("rounds", [-1, 1])
+@pytest.mark.parametrize("speed", [2000.0, 600.0, 300.0, 100.0])
+def test_hot_ensemble(rounds, speed):
+    """Re-sorts every step, every few steps and every dozen: rounds that stop
+    early, short ones, and IF nodes."""
+    n, rng = 500, np.random.default_rng(5)
+    g = np.arange(n)
+    pos = np.stack([g % 8, g // 8 % 8, g // 64], 1) * 0.45 + 0.3
+    S = synth.box_system(n, 3.9, 3.9, 0.45, 0, density=2500e-6, kn=1e6, restitution=0.9, mu=0.3)
+    W = synth.box_walls(3.9, 3.9)
+    vel = rng.normal(scale=speed, size=pos.shape).astype(np.float32)
+    ens = E.Ensemble([S], W, law=E.LAW_LINEAR, dt=5e-6, skin=0.02, use_graph=1)
+    ens.set_launch(rounds=rounds)
+    o = EnsRestated([S], W, E.LAW_LINEAR, 5e-6, 0.02, 32, precision="f32")
+    for e in (ens, o):
+        e.set_state(pos.astype(np.float32), np.full(n, 0.2, np.float32), vel)
+        for k in (33, 8, 64, 17, 20):
+            e.step(k)
+    a, b = ens.state(), o.state()
+    assert a["status"] == b["status"]
+    assert ens.num_rebuilds() == o.num_rebuilds() > 4
+    for k in ("pos", "vel", "avel"):
+        np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
+    ens.close()
+    o.close()
+
+
+@pytest.mark.parametrize("n", [200001, 1 << 20, (1 << 20) + 1])
+def test_graph_kind_by_size(n):
+    """The largest box in rounds and the smallest with IF nodes; and a size
+    between them (a cylinder around it: IF nodes, the box alone: rounds)."""
+    S, W, pos, rad, vel = ens_box(n)
+    if n == 200001:
+        c = 0.5 * float(pos[:, 0].max() + 0.2)
+        W = W + [E.cylinder((c, c, 0.0), (0.0, 0.0, 1.0), 3.0 * c)]
+        S[0].nwalls = 7
+    out = []
+    for g in (0, 1):
+        e = E.Ensemble(S, W, law=E.LAW_LINEAR, dt=5e-6, skin=0.02, use_graph=g)
+        e.set_state(pos, rad, vel)
+        for k in (9, 8):
+            e.step(k)
+        out.append((e.state(), e.num_rebuilds()))
+        e.close()
+    assert out[0][0]["status"] == out[1][0]["status"] == 0 and out[0][1] == out[1][1] > 1
+    for k in ("pos", "vel", "avel", "pid"):
+        np.testing.assert_array_equal(out[0][0][k], out[1][0][k], err_msg=k)
