@@ -537,13 +537,34 @@ int add_conditional(cudaStream_t cs, cudaGraphConditionalHandle h,
   return 0;
 }
 
+// A graph being captured: whichever way its builder returns, no capture stays
+// open, the graph is destroyed and the state buffer is the one of before.
+struct GraphBuild {
+  blaze_ens* e;
+  const int cur;
+  cudaGraph_t g = nullptr;
+  explicit GraphBuild(blaze_ens* x) : e(x), cur(x->cur) {}
+  GraphBuild(const GraphBuild&) = delete;
+  GraphBuild& operator=(const GraphBuild&) = delete;
+  ~GraphBuild() {
+    for (cudaStream_t st : {e->aux2, e->aux, e->stream}) {   // inner captures first
+      cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+      cudaGraph_t part = nullptr;
+      if (cudaStreamIsCapturing(st, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone)
+        cudaStreamEndCapture(st, &part);
+    }
+    if (g) cudaGraphDestroy(g);
+    e->cur = cur;
+  }
+};
+
 // kGraphSteps steps as one graph starting from S[c]: a gate kernel carries
 // the pending re-sort request into the first step's IF node; each step kernel
 // sets the next step's IF condition when any particle has moved half the skin.
 int build_if_graph(blaze_ens* e, int c) {
-  const int saved = e->cur;
+  GraphBuild build(e);
+  cudaGraph_t& g = build.g;
   e->cur = c;
-  cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
   cudaGraphConditionalHandle h[kGraphSteps];
   for (int k = 0; k < kGraphSteps; ++k)
@@ -571,8 +592,6 @@ int build_if_graph(blaze_ens* e, int c) {
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(e->stream, &out));
   CK(cudaGraphInstantiate(&e->graph[c], out, 0));
-  CK(cudaGraphDestroy(out));
-  e->cur = saved;
   return 0;
 }
 
@@ -610,9 +629,9 @@ bool in_rounds(const blaze_ens* e) {
   return e->n <= (e->curved || e->npoly > 0 ? kRoundMaxCurved : kRoundMax);
 }
 int build_round_graph(blaze_ens* e, int c) {
-  const int saved = e->cur;
+  GraphBuild build(e);
+  cudaGraph_t& g = build.g;
   const EnsRound r = round_words(e);
-  cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
   cudaGraphConditionalHandle hw;
   CK(cudaGraphConditionalHandleCreate(&hw, g, 1, cudaGraphCondAssignDefault));
@@ -651,8 +670,6 @@ int build_round_graph(blaze_ens* e, int c) {
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(e->stream, &out));
   CK(cudaGraphInstantiate(&e->graph[c], out, 0));
-  CK(cudaGraphDestroy(out));
-  e->cur = saved;
   return 0;
 }
 
@@ -1701,9 +1718,9 @@ int restore_checkpoint(blaze_ens_adj* a, const EnsCheckpoint& c) {
 // re-sort), then the tape tick and the recording step.
 int build_record_graph(blaze_ens_adj* a, int c) {
   blaze_ens* e = a->e;
-  const int saved = e->cur;
+  GraphBuild build(e);
+  cudaGraph_t& g = build.g;
   e->cur = c;
-  cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
   cudaGraphConditionalHandle h[kGraphSteps];
   for (int k = 0; k < kGraphSteps; ++k)
@@ -1712,26 +1729,13 @@ int build_record_graph(blaze_ens_adj* a, int c) {
                                    cudaStreamCaptureModeThreadLocal));
   launch_gate_graph(e->ctl, h[0], e->d_rb, kGraphSteps, e->stream);
   for (int k = 0; k < kGraphSteps; ++k) {
-    cudaStreamCaptureStatus cs;
-    cudaGraph_t capg = nullptr;
-    const cudaGraphNode_t* deps = nullptr;
-    size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(e->stream, &cs, nullptr, &capg, &deps, &ndeps));
-    alignas(cudaGraphNodeParams) unsigned char raw[sizeof(cudaGraphNodeParams)];
-    std::memset(raw, 0, sizeof(raw));
-    cudaGraphNodeParams& cp = *reinterpret_cast<cudaGraphNodeParams*>(raw);
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = h[k];
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    CK(cudaGraphAddNode(&cnode, capg, deps, ndeps, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CK(cudaStreamUpdateCaptureDependencies(e->stream, &cnode, 1, cudaStreamSetCaptureDependencies));
+    cudaGraph_t body = nullptr;
+    int rc = add_conditional(e->stream, h[k], cudaGraphCondTypeIf, &body);
+    if (rc) return rc;
     CK(cudaStreamBeginCaptureToGraph(e->aux, body, nullptr, nullptr, 0,
                                      cudaStreamCaptureModeThreadLocal));
     CK(cudaMemsetAsync(e->d_rb + k, 0x01, sizeof(int), e->aux));
-    int rc = enqueue_rebuild(e, nullptr, e->aux);
+    rc = enqueue_rebuild(e, nullptr, e->aux);
     adj_launch_list(e->b, a->tape, e->n, e->ctl, nullptr, 1, e->cs.perm, e->aux);
     cudaGraph_t tmp = nullptr;
     CK(cudaStreamEndCapture(e->aux, &tmp));
@@ -1746,8 +1750,6 @@ int build_record_graph(blaze_ens_adj* a, int c) {
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(e->stream, &out));
   CK(cudaGraphInstantiate(&a->rgraph[c], out, 0));
-  CK(cudaGraphDestroy(out));
-  e->cur = saved;
   return 0;
 }
 
