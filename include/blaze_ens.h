@@ -135,8 +135,10 @@ int blaze_ens_num_rebuilds(blaze_ens* e);
 /* Device pointers of the current state (float4 pos+radius, vel+bits,
  * angular velocity+path) and the ensemble's CUDA stream. */
 int blaze_ens_device_state(blaze_ens* e, void** pos4, void** vel4, void** angv4, void** stream);
-/* Kernels launched by the last blaze_ens_step that always run (re-sorts are
- * counted by blaze_ens_rebuild_kernels each). */
+/* Kernels of the last blaze_ens_step without its re-sorts, each of which adds
+ * blaze_ens_rebuild_kernels: with graph stepping in rounds also the round that
+ * a re-sort starts.  Launches of a round that find nothing to do (the steps
+ * behind one that asks for a re-sort) are not counted. */
 int blaze_ens_last_launches(blaze_ens* e);
 int blaze_ens_rebuild_kernels(blaze_ens* e);
 /* Profiling: while on, blaze_ens_step runs plain steps, each waiting for the

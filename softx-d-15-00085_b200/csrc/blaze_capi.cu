@@ -79,7 +79,10 @@ struct blaze_sim {
   // (block start, check after the step) (build_single)
   cudaGraphExec_t block[2] = {nullptr, nullptr};
   cudaGraphExec_t single[2][2][2] = {};
-  int step_launches = 0;               // kernels of one step, counted when a graph is built
+  // step kernels of a graph of kGraphSteps steps and of a single step, counted
+  // when the graph is built (with energy tallies a graph's later steps need no
+  // kernel for the volume objects' moves)
+  int graph_launches = 0, single_launches = 0;
   int* d_rb = nullptr;                 // per graph step: nonzero when that step re-sorted
   uint32_t* d_chk = nullptr;           // list-check maxima slots (StepCtl::chk)
   bool spin_free = false;              // rotation off and every angular velocity zero
@@ -825,17 +828,18 @@ int add_rebuild_if(blaze_sim* s, cudaStream_t cs, cudaStream_t bs, cudaGraphCond
 // call of one step of 10,000 spheres 24.9 -> 19.7 us (three states at once; one
 // alone 74 -> 60), against a gate kernel and separate launches.
 int build_graph(blaze_sim* s, int c, int steps, cudaGraphExec_t* out_exec) {
-  const int saved = s->cur, launches = s->last_launches;
+  const int saved = s->cur;
   s->cur = c;
   cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
   CK(cudaStreamBeginCaptureToGraph(s->stream, g, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
+  int& count = steps == 1 ? s->single_launches : s->graph_launches;
+  count = 0;
   for (int k = 0; k < steps; ++k) {
     enqueue_reference_rebuild(s, s->stream);
-    const int ks = enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream, k == 0,
-                                        k + 1 == steps);
-    if (k == 0) s->step_launches = ks;
+    count += enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream, k == 0,
+                                  k + 1 == steps);
     s->cur ^= 1;
   }
   cudaGraph_t out = nullptr;
@@ -843,7 +847,6 @@ int build_graph(blaze_sim* s, int c, int steps, cudaGraphExec_t* out_exec) {
   CK(cudaGraphInstantiate(out_exec, out, 0));
   CK(cudaGraphDestroy(out));
   s->cur = saved;
-  s->last_launches = launches;
   return 0;
 }
 
@@ -868,13 +871,14 @@ int capture_block_body(blaze_sim* s, cudaGraph_t body, cudaStream_t bs, cudaStre
   CK(cudaStreamBeginCaptureToGraph(bs, body, nullptr, nullptr, 0,
                                    cudaStreamCaptureModeThreadLocal));
   int rc = 0;
+  s->graph_launches = 0;   // the same for the three kinds
   if (kind == kBlockResort) rc = enqueue_rebuild(s, nullptr, bs);
   if (kind == kBlockExact) launch_gate_body(s->ctl, h[0], bs);
   for (int k = 0; k < kGraphSteps && !rc; ++k) {
     if (k < n_if) rc = add_rebuild_if(s, bs, bs2, h[k], k);
     const StepLink link = k + 1 < n_if ? StepLink{s->d_rb + k, h[k + 1], 1, 0}
                                         : StepLink{s->d_rb + k, 0, 0, (int)(k + 1 == kGraphSteps)};
-    s->step_launches = enqueue_step_kernels(s, link, bs, k == 0, k + 1 == kGraphSteps);
+    s->graph_launches += enqueue_step_kernels(s, link, bs, k == 0, k + 1 == kGraphSteps);
     s->cur ^= 1;
   }
   cudaGraph_t tmp = nullptr;
@@ -921,8 +925,8 @@ int build_single(blaze_sim* s, int c, int bstart, int chk) {
                                    cudaStreamCaptureModeThreadLocal));
   launch_gate_if(s->ctl, h, s->opt.skin, list_look(s), bstart, wall_speed(s), s->stream);
   int rc = add_rebuild_if(s, s->stream, s->aux, h, -1);
-  if (!rc) s->step_launches = enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, chk},
-                                                   s->stream);
+  if (!rc) s->single_launches = enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, chk},
+                                                     s->stream);
   cudaGraph_t out = nullptr;
   CK(cudaStreamEndCapture(s->stream, &out));
   if (!rc) CK(cudaGraphInstantiate(&s->single[c][bstart][chk], out, 0));
@@ -963,6 +967,7 @@ int prepare_graphs(blaze_sim* s) {
 int graph_steps(blaze_sim* s, int nsteps) {
   int rc = prepare_graphs(s);
   if (rc) return rc;
+  s->last_launches = 0;   // what a capture enqueued has not run
   int done = 0;
   while (done < nsteps) {
     // a removal check every 1000 steps ends a step outside a block
@@ -973,14 +978,14 @@ int graph_steps(blaze_sim* s, int nsteps) {
         CK(cudaGraphLaunch(s->block[c], s->stream));
         // the gate and the step kernels (re-sorts and the exact mode's
         // extra gate are counted on the device)
-        s->last_launches += 1 + kGraphSteps * s->step_launches;
+        s->last_launches += 1 + s->graph_launches;
         s->steps += kGraphSteps;
         if (s->si.Kill_Particles) s->stepc += kGraphSteps;
         if (kGraphSteps & 1) s->cur ^= 1;
         done += kGraphSteps;
       } else {
         CK(cudaGraphLaunch(s->single[c][block_start_here(s)][check_after_here(s)], s->stream));
-        s->last_launches += 1 + s->step_launches;
+        s->last_launches += 1 + s->single_launches;
         finish_step(s);
         done += 1;
       }
@@ -989,13 +994,13 @@ int graph_steps(blaze_sim* s, int nsteps) {
     // launches besides the re-sorts, which blaze_num_rebuilds counts
     if (nsteps - done < kGraphSteps || kill_soon) {
       CK(cudaGraphLaunch(s->single[c][0][0], s->stream));
-      s->last_launches += s->step_launches;
+      s->last_launches += s->single_launches;
       finish_step(s);
       done += 1;
       continue;
     }
     CK(cudaGraphLaunch(s->graph[c], s->stream));
-    s->last_launches += kGraphSteps * s->step_launches;
+    s->last_launches += s->graph_launches;
     s->steps += kGraphSteps;
     if (s->si.Kill_Particles) s->stepc += kGraphSteps;
     if (kGraphSteps & 1) s->cur ^= 1;

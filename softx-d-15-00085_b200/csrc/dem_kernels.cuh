@@ -48,9 +48,6 @@ struct NbrList {
   int* flat_n;          // entries in `flat` (reset before each rebuild)
 };
 
-// How a step learns whether it consumes a fresh re-sort, and how it asks for
-// the next one: through StepCtl (plain stepping) or, inside a CUDA graph,
-// through the IF-node condition of the next step.
 // An ensemble's round of steps (graph stepping): the steps of a round are
 // launched in a row, and a step does nothing when an earlier one of the round
 // has asked for a re-sort (k > *stop) or the call's steps are done (k >=
@@ -61,6 +58,9 @@ struct RoundLink {
   int k;             // this step's index in the round
 };
 
+// How a step learns whether it consumes a fresh re-sort, and how it asks for
+// the next one: through StepCtl (plain stepping) or, inside a CUDA graph,
+// through the IF-node condition of the next step.
 struct StepLink {
   const int* rebuilt;                  // nonzero: read the sorted buffer
   cudaGraphConditionalHandle next_h;   // next step's IF condition (graph)

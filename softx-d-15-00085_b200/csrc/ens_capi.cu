@@ -1081,16 +1081,21 @@ int blaze_ens_get_state(blaze_ens* e, float* pos3, float* radius, float* vel3, f
 
 namespace {
 
+// Persistent stepping (no drum turns: those advance between steps), where every
+// particle has a lane of the resident grid.  The step kernel's own grid is faster
+// beyond that (in rounds, boxes settling from rest, us a step: 160,000 spheres
+// 10.8 against 9.9, 400,000 17.3 against 16.3; three side by side 16.9 against
+// 7.6 and 25.2 against 18.3).
+bool persists(const blaze_ens* e) {
+  return e->opt.use_graph == 2 && !e->opt.capture_forces && !e->any_rot && e->npoly == 0 &&
+         e->n <= kEnsOneWave;
+}
+
 // nsteps steps, as CUDA graphs where `graphs` allows; what is left of a call
 // after its graphs, fewer than kGraphSteps steps, as plain steps (a round of
 // so few would mostly be launches that do nothing).
 int advance(blaze_ens* e, int nsteps, bool graphs) {
-  // persistent stepping (no drum turns: those advance between steps), where
-  // every particle has a lane of the resident grid; beyond that the step
-  // kernel's own grid is faster (400,000 spheres 121 against 105 us a step,
-  // boxes of 2,000,000 450 against 400)
-  if (graphs && e->opt.use_graph == 2 && !e->opt.capture_forces && !e->any_rot && e->npoly == 0 &&
-      nsteps > 0 && e->n <= kEnsOneWave) {
+  if (graphs && persists(e) && nsteps > 0) {
     const int c = e->cur;
     if (!e->pgraph[c]) {
       int rc = build_persist_graph(e, c);
@@ -1109,8 +1114,9 @@ int advance(blaze_ens* e, int nsteps, bool graphs) {
     }
     ens_launch_round_init(round_words(e), nsteps, c, e->stream);
     CK(cudaGraphLaunch(e->graph[c], e->stream));
-    const int rounds = (nsteps + kRoundSteps - 1) / kRoundSteps;   // with no re-sort
-    e->last_launches += 2 + rounds * (2 + kRoundSteps * step_kernel_count(e));
+    // the kernels of the steps, and the rounds' own, as many as with no re-sort
+    const int rounds = (nsteps + kRoundSteps - 1) / kRoundSteps;
+    e->last_launches += 2 + 2 * rounds + nsteps * step_kernel_count(e);
     e->cur ^= nsteps & 1;
     return 0;
   }
@@ -1248,8 +1254,10 @@ int blaze_ens_last_launches(blaze_ens* e) { return e ? e->last_launches : -1; }
 
 int blaze_ens_rebuild_kernels(blaze_ens* e) {
   if (!e) return -1;
-  // persistent stepping: a re-sort also starts another round (gate + step)
-  return rebuild_kernel_count(e) + (e->opt.use_graph == 2 && e->n <= kEnsOneWave ? 2 : 0);
+  // a re-sort also starts another round: its gate and its step kernel (persistent)
+  // or end
+  const bool round = e->opt.use_graph != 0 && !e->prof && (persists(e) || in_rounds(e));
+  return rebuild_kernel_count(e) + (round ? 2 : 0);
 }
 
 }  // extern "C"

@@ -293,3 +293,31 @@ def test_graph_kind_by_size(n):
     assert out[0][0]["status"] == out[1][0]["status"] == 0 and out[0][1] == out[1][1] > 1
     for k in ("pos", "vel", "avel", "pid"):
         np.testing.assert_array_equal(out[0][0][k], out[1][0][k], err_msg=k)
+
+
+def test_launch_counts(tmp_path):
+    """The launches that a step call reports, by what runs it."""
+    P, st = synth.mill_project(str(tmp_path), n=3000)
+    axis = float(P.wobj[0].cyl_geo.radius)
+    s = device.Simulation(P, skin=0.05, use_graph=1)
+    s.set_cylinder_rotation(True)
+    s.set_state(st["pos"], st["vel"], st["avel"], st["type"], st["pid"])
+    s.set_dobj_rotation(axis, axis, float(P.mill.RadPerStep))
+    s.step(8)                       # after a new state: a gate, a move and a step each
+    assert s.last_launches() == 8 * 3
+    s.step(16)                      # two blocks: a gate, a move and eight steps
+    assert s.last_launches() == 2 * (1 + 1 + 8)
+    s.step(3)
+    assert s.last_launches() == 3 * 3
+    s.close()
+    S, W, pos, rad, vel = ens_box(500)
+    for graph, rounds, capture, steps, resort in ((0, 0, 0, 40 * 7, 5), (1, 1, 0, 2 + 6 + 40, 7),
+                                                  (1, -1, 0, 5 * 9, 5), (2, 0, 0, 3, 7),
+                                                  (2, 0, 1, 2 + 6 + 40, 7), (2, -1, 1, 5 * 9, 5)):
+        e = E.Ensemble(S, W, law=E.LAW_LINEAR, dt=5e-6, skin=0.02, use_graph=graph,
+                       capture_forces=capture)
+        e.set_launch(rounds=rounds)
+        e.set_state(pos, rad)
+        e.step(40)
+        assert (e.last_launches(), e.rebuild_kernels()) == (steps, resort), (graph, rounds, capture)
+        e.close()
