@@ -240,6 +240,7 @@ k_nlist(const SimParams* __restrict__ P, const float4* __restrict__ pos, int n_m
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) ctl->epoch += 1;
   const int n = ctl->n_cur;
+  const unsigned live = __ballot_sync(0xffffffffu, i < n);   // a prefix of the warp
   if (i >= n) return;
   const float4 pa4 = pos[i];
   const float3 pa = xyz(pa4);
@@ -315,19 +316,19 @@ k_nlist(const SimParams* __restrict__ P, const float4* __restrict__ pos, int n_m
   const uint32_t kept = cnt < (uint32_t)nl.cap ? cnt : (uint32_t)nl.cap;
   nl.cnt[i] = kept;
   if (nl.flat) {
-    // append this particle's slots to the flat list: one atomic per warp;
-    // the lanes still here (i < n) are a prefix of the warp
-    const unsigned m = __activemask();
+    // append this particle's slots to the flat list: one atomic per warp.  The
+    // lanes' searches end one by one, so the mask is the one from before them:
+    // every live lane comes here.
     const int lane = threadIdx.x & 31;
     uint32_t x = kept;
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t y = __shfl_up_sync(m, x, d);
+      const uint32_t y = __shfl_up_sync(live, x, d);
       if (lane >= d) x += y;
     }
-    const int last = 31 - __clz((int)m);
+    const int last = 31 - __clz((int)live);
     uint32_t base = 0;
     if (lane == last) base = (uint32_t)atomicAdd(nl.flat_n, (int)x);
-    base = __shfl_sync(m, base, last) + (x - kept);
+    base = __shfl_sync(live, base, last) + (x - kept);
     for (uint32_t k = 0; k < kept; ++k) nl.flat[base + k] = k * (uint32_t)nl.stride + (uint32_t)i;
   }
   flag_status(ctl, st);
