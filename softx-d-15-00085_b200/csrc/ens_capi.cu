@@ -331,7 +331,8 @@ void build_tri_lists(const blaze_ens* e, std::vector<uint32_t>& off, std::vector
 
 // A sphere around triangle W: about the middle of its longest edge or its
 // centroid, whichever gives the smaller one, with the radius rounded up by
-// 1e-5 of the coordinates' size (the FP32 distance tests round at 1e-7).
+// 1e-5 of the coordinates' size (the centre rounds at 6e-8 of it); the tests
+// against it add their own margin for the sphere's radius.
 float4 tri_bound(const EnsWallDev& W) {
   const double v[3][3] = {{W.a.x, W.a.y, W.a.z}, {W.b.x, W.b.y, W.b.z}, {W.c.x, W.c.y, W.c.z}};
   auto dist = [](const double* p, const double* q) {

@@ -743,10 +743,13 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
         float delta = 0.0f;
         if (q < c1) {
           // most of a cell's triangles are out of reach: a sphere around each
-          // tells (rounded up by more than the test's own rounding, tri_bound)
+          // (tri_bound) tells.  Its radius is rounded up by the coordinates'
+          // size, the sum by 1e-6: the FP32 distance and square are off by 2e-7
+          // of the sum, which a large sphere at a small mesh near the origin
+          // would see.
           const float4 bs = __ldg(g.stri_b + q);
           const float3 dc = pp - xyz(bs);
-          const float reach = bs.w + rp;
+          const float reach = (bs.w + rp) * (1.0f + 1e-6f);
           float3 nrm;
           if (!(dot3(dc, dc) > reach * reach))
             hit = wall_touch<kCurved>(g.walls[__ldg(g.stri_ids + q)], pp, rp, nrm, delta, region);

@@ -321,3 +321,44 @@ def test_launch_counts(tmp_path):
         e.step(40)
         assert (e.last_launches(), e.rebuild_kernels()) == (steps, resort), (graph, rounds, capture)
         e.close()
+
+
+# (size of the triangle, radius, centre): spheres that touch a vertex of a small
+# triangle at the origin by a few 1e-8 cm, where FP32 rounds the distance to the
+# triangle's bounding sphere beyond the sum of the radii
+GRAZING = [
+    (0.0012349095360439084, 1.4137132167816162, (1.4149479866027832, -0.00039765366818755865, 0.00037886638892814517)),
+    (0.0013415310415354174, 1.9994114637374878, (2.0007522106170654, 0.0010979132493957877, 0.0013439931208267808)),
+    (0.0025264999515147773, 1.4134680032730103, (1.4159938097000122, 0.0010431538103148341, 0.000926253735087812)),
+    (0.0002965804566498865, 1.999942421913147, (2.0002386569976807, 0.0009980620816349983, -0.0005503043648786843)),
+    (0.0007389509463619639, 1.999290943145752, (2.0000290870666504, -0.0016199497040361166, 0.0005662687472067773)),
+    (6.981820006969034e-05, 0.49996626377105713, (0.5000360608100891, -0.0001299064460908994, -1.1633491340035107e-05)),
+    (5.280388288221428e-05, 0.9999672770500183, (1.0000196695327759, 0.000817042775452137, 0.00034754013177007437)),
+    (6.595577163958962e-05, 0.9999799728393555, (1.0000455379486084, -0.0008272947743535042, 0.0002528926415834576)),
+]
+
+
+def test_grazing_contact_with_a_small_triangle():
+    S, W, pos, rad = [], [], [], []
+    for k, (s, r, p) in enumerate(GRAZING):
+        W.append(E.triangle((s, 0, 0), (-0.5 * s, 0.8 * s, 0), (-0.5 * s, -0.8 * s, 0)))
+        y = synth.box_system(1, 8.0, 8.0, 4.1, 0, density=2500e-6, kn=1e8, restitution=0.6,
+                             mu=0.4, gravity=(0.0, 0.0, 0.0))
+        y.nwalls, y.tri0, y.ntris = 0, k, 1
+        for a in range(3):
+            y.origin[a] = -4.1
+        S.append(y)
+        pos.append(p)
+        rad.append(r)
+    pos, rad = np.array(pos, np.float32), np.array(rad, np.float32)
+    ens = E.Ensemble(S, W, law=E.LAW_LINEAR, dt=1e-4, skin=0.01, use_graph=0)
+    o = EnsRestated(S, W, E.LAW_LINEAR, 1e-4, 0.01, 32, precision="f32")
+    for e in (ens, o):
+        e.set_state(pos, rad)
+        e.step(1)
+    a, b = ens.state(), o.state()
+    assert a["status"] == b["status"] == 0
+    assert (b["vel"][:, 0] > 0).all()
+    np.testing.assert_array_equal(a["vel"].astype(np.float64), b["vel"])
+    ens.close()
+    o.close()
