@@ -219,6 +219,7 @@ void build_params(blaze_sim* s) {
       G.edge1[e] = (int)(D.edge[e].point_vindex[1] & 7u);
     }
   }
+  P.n_ops = (int)s->ops.size();   // the wall program stays (upload_walls replaces it)
   P.max_nbr = s->opt.max_nbr;
   P.skin = s->opt.skin;
   // The neighbour search may skip cells out of a particle's reach only where

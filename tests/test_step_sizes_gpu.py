@@ -362,3 +362,27 @@ def test_grazing_contact_with_a_small_triangle():
     np.testing.assert_array_equal(a["vel"].astype(np.float64), b["vel"])
     ens.close()
     o.close()
+
+
+@pytest.mark.parametrize("grid", [0, 1])
+def test_new_volume_objects_keep_the_world_objects(tmp_path, grid):
+    """blaze_update_dobj replaces the volume objects and nothing else: without
+    the per-cell wall lists (also with polyhedra, or moving walls) the particles
+    lost every world object."""
+    r, n = 0.1, 257
+    P, _ = synth.box_project(str(tmp_path), n_side=(2, 2, 2), radius=r)
+    P.sim_info.Num_Particles = n
+    pos, rng, _ = lattice(n, 0.1995, 0.0995, n)       # touching the walls and each other
+    vel = rng.normal(scale=10.0, size=(n, 3)).astype(np.float32)
+    avel, ty, pid = np.zeros_like(vel), np.zeros(n, np.uint32), np.arange(n, dtype=np.int32)
+    sim = device.Simulation(P, wall_grid=grid)
+    ref = Restated("f32").init(P.sim_info, P.wobj, P.n_w, P.pobj, P.n_p, P.dobj, P.n_d)
+    for s in (sim, ref):
+        s.set_state(pos, vel, avel, ty, pid)
+    sim.update_dobj(P.dobj, P.n_d)
+    sim.step(5)
+    ref.step(5)
+    a, b = sim.state(), ref.state()
+    for k in ("pos", "vel", "avel"):
+        np.testing.assert_array_equal(a[k].astype(np.float64), b[k], err_msg=k)
+    sim.close()
