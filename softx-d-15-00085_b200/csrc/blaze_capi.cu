@@ -53,6 +53,7 @@ struct blaze_sim {
   int cyl_rot = 0;
   SimParams hp{};
   SimParams* dp = nullptr;
+  SimParams* dp2 = nullptr;   // second copy (enqueue_step_kernels)
   std::vector<WallOp> ops;
   WallOp* d_ops = nullptr;
   uint32_t* d_wall_off = nullptr;
@@ -377,6 +378,16 @@ void build_wall_grid(blaze_sim* s, std::vector<uint32_t>& off, std::vector<uint1
   off[nt] = (uint32_t)idx.size();
 }
 
+// The parameters to the device, both copies (enqueue_step_kernels).
+cudaError_t send_params(blaze_sim* s) {
+  for (SimParams* d : {s->dp, s->dp2}) {
+    const cudaError_t e =
+        cudaMemcpyAsync(d, &s->hp, sizeof(SimParams), cudaMemcpyHostToDevice, s->stream);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 // With the volume objects turned on the device, copy them back into the
 // host's DOBJ and parameter mirrors (vertices, faces, centre of mass) before
 // anything re-uploads the parameters from the host.
@@ -433,7 +444,7 @@ int upload_walls(blaze_sim* s) {
   if (rc) return rc;
   drop_graphs(s);
   build_ops(s);
-  CK(cudaMemcpyAsync(s->dp, &s->hp, sizeof(SimParams), cudaMemcpyHostToDevice, s->stream));
+  CK(send_params(s));
   if (s->d_ops) CK(cudaFree(s->d_ops));
   s->d_ops = nullptr;
   CK(dalloc(&s->d_ops, s->ops.size()));
@@ -600,17 +611,21 @@ cudaEvent_t prof_event(blaze_sim* s, int phase) {
 // The kernels of one step after the (conditional) re-sort, reading S[cur]
 // or the sorted copy S[2] as `link` says and writing S[cur ^ 1]; returns the
 // number of launches.
-// first / last: of the steps launched together (a graph's); with energy
-// tallies the step before moves a step's volume objects (StepTail::next).
-int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st, bool first = true,
-                         bool last = true) {
+// Step `at` of `steps` launched together (a graph's): with energy tallies the
+// step before moves a step's volume objects (StepTail::next), from one copy of
+// the parameters to the other, so that no kernel writes what it reads; the last
+// step reads the first copy, which is then the current one.
+int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st, int at = 0,
+                         int steps = 1) {
   const ForceCapture* cap = s->opt.capture_forces ? &s->cap : nullptr;
   int k = 1;
   const bool moves = (s->dobj_rot || s->dobj_tr >= 0) && s->n_d > 0;
   const DobjMove mv{s->dobj_rot ? 1 : 0, s->dobj_tr, s->rot_ax, s->rot_ay, s->rot_c, s->rot_s};
   const bool energy = s->hp.energy_calc && s->d_epart;   // allocated when EnergyCalc
-  if (moves && (first || s->poly || !energy)) {
-    launch_move_dobj(s->dp, mv, s->n_d, st);
+  const bool chain = moves && energy && !s->poly;
+  SimParams* dp = chain && ((steps - 1 - at) & 1) ? s->dp2 : s->dp;
+  if (moves && (at == 0 || !chain)) {
+    launch_move_dobj(s->dp, dp, mv, s->n_d, st);
     ++k;
   }
   if (s->wobj_rot) {
@@ -629,8 +644,9 @@ int enqueue_step_kernels(blaze_sim* s, StepLink link, cudaStream_t st, bool firs
                      st);
     k += 1 + np;
   } else {
-    const StepTail tail{s->d_done, s->d_epart, s->d_tally, s->dp, mv, moves && !last ? 1 : 0};
-    launch_step(s->dp, s->d_ops, WallGrid{s->d_wall_off, s->d_wall_idx}, s->S[s->cur], s->S[2],
+    SimParams* next = chain && at + 1 < steps ? (dp == s->dp ? s->dp2 : s->dp) : nullptr;
+    const StepTail tail{s->d_done, s->d_epart, s->d_tally, next, mv};
+    launch_step(dp, s->d_ops, WallGrid{s->d_wall_off, s->d_wall_idx}, s->S[s->cur], s->S[2],
                 s->S[s->cur ^ 1], s->ob, s->n_max, s->nl, s->ctl, link, s->spin_free, cap, energy,
                 tail, s->opt.fast_law != 0, st);
   }
@@ -839,8 +855,8 @@ int build_graph(blaze_sim* s, int c, int steps, cudaGraphExec_t* out_exec) {
   count = 0;
   for (int k = 0; k < steps; ++k) {
     enqueue_reference_rebuild(s, s->stream);
-    count += enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream, k == 0,
-                                  k + 1 == steps);
+    count += enqueue_step_kernels(s, StepLink{&s->ctl->rebuilt, 0, 0, 1}, s->stream, k,
+                                  steps);
     s->cur ^= 1;
   }
   cudaGraph_t out = nullptr;
@@ -879,7 +895,7 @@ int capture_block_body(blaze_sim* s, cudaGraph_t body, cudaStream_t bs, cudaStre
     if (k < n_if) rc = add_rebuild_if(s, bs, bs2, h[k], k);
     const StepLink link = k + 1 < n_if ? StepLink{s->d_rb + k, h[k + 1], 1, 0}
                                         : StepLink{s->d_rb + k, 0, 0, (int)(k + 1 == kGraphSteps)};
-    s->graph_launches += enqueue_step_kernels(s, link, bs, k == 0, k + 1 == kGraphSteps);
+    s->graph_launches += enqueue_step_kernels(s, link, bs, k, kGraphSteps);
     s->cur ^= 1;
   }
   cudaGraph_t tmp = nullptr;
@@ -1089,7 +1105,8 @@ void free_sim(blaze_sim* s) {
   for (int b = 0; b < 2; ++b) { f(s->ob.pid[b]); f(s->ob.lift[b]); }
   f(s->cs.key); f(s->cs.slot); f(s->cs.member); f(s->cs.cnt); f(s->cs.start); f(s->cs.tile);
   f(s->cs.spec); f(s->d_done); f(s->nl.idx); f(s->nl.cnt);
-  f(s->ctl); f(s->d_rb); f(s->d_chk); f(s->dp); f(s->d_ops); f(s->d_wall_off); f(s->d_wall_idx);
+  f(s->ctl); f(s->d_rb); f(s->d_chk); f(s->dp); f(s->dp2);
+  f(s->d_ops); f(s->d_wall_off); f(s->d_wall_idx);
   f(s->d_tally); f(s->d_eb); f(s->d_epart);
   f(s->cap.f_pp); f(s->cap.t_pp); f(s->cap.f_w); f(s->cap.t_w); f(s->cap.f_l); f(s->cap.t_l);
   if (s->h_ctl) cudaFreeHost(s->h_ctl);
@@ -1252,6 +1269,7 @@ int create_impl(blaze_sim** out, const WOBJ* w, int n_w, const POBJ* p, int n_p,
   CKF(dalloc(&s->cs.member, n));
   CKF(dalloc(&s->cs.spec, (size_t)2 * sort_blocks(n)));
   CKF(dalloc(&s->dp, 1));
+  CKF(dalloc(&s->dp2, 1));
   CKF(dalloc(&s->ctl, 1));
   CKF(dalloc(&s->d_rb, kGraphSteps));
   CKF(cudaMemset(s->d_rb, 0, sizeof(int) * kGraphSteps));
@@ -1367,7 +1385,7 @@ int blaze_set_cylinder_rotation(blaze_sim* s, int on) {
   s->cyl_rot = on ? 1 : 0;
   s->hp.cyl_rot = s->cyl_rot;
   drop_graphs(s);   // the list check's wall speed changes
-  CK(cudaMemcpyAsync(s->dp, &s->hp, sizeof(SimParams), cudaMemcpyHostToDevice, s->stream));
+  CK(send_params(s));
   CK(cudaStreamSynchronize(s->stream));
   return 0;
 }
@@ -1466,7 +1484,7 @@ int blaze_update_dobj(blaze_sim* s, const DOBJ* d, int n_d) {
   std::memcpy(s->d, d, sizeof(DOBJ) * n_d);
   s->dobj_on_device = false;   // the caller's objects replace the turned ones
   build_params(s);
-  CK(cudaMemcpyAsync(s->dp, &s->hp, sizeof(SimParams), cudaMemcpyHostToDevice, s->stream));
+  CK(send_params(s));
   CK(cudaStreamSynchronize(s->stream));
   return 0;
 }

@@ -472,28 +472,38 @@ __device__ void dobj_face(DobjDev& D, int j) {
 // moves by its velocity times dt.  A block's threads share the vertices, then
 // the faces (an object's faces are formed once, from its final vertices; the
 // functions would form them after each move and read only the last).
-__device__ void move_dobjs(SimParams* P, const DobjMove& mv) {
+// From src into dst, which may be the same and otherwise holds the same objects
+// (every vertex, centre and face is written).
+__device__ void move_dobjs(const SimParams* src, SimParams* dst, const DobjMove& mv) {
   const float3 about = f3(mv.ax, mv.ay, 0.0f);
-  const int n = P->n_dobj;
+  const int n = src->n_dobj;
   for (int t = threadIdx.x; t < 9 * n; t += blockDim.x) {   // 8 vertices and the centre
-    DobjDev& D = P->dobj[t / 9];
+    const DobjDev& D = src->dobj[t / 9];
     const int k = t % 9;
     if (k < 8 && k >= D.num_vertex) continue;
     float3 v = k < 8 ? D.vert[k] : D.com;
     if (mv.turn && D.attached) v = turn_about(v, about, mv.c, mv.s);
-    if (t / 9 == mv.tr) v = v + D.velocity * P->dt;
-    if (k < 8) D.vert[k] = v;
-    else D.com = v;
+    if (t / 9 == mv.tr) v = v + D.velocity * src->dt;
+    if (k < 8) dst->dobj[t / 9].vert[k] = v;
+    else dst->dobj[t / 9].com = v;
   }
   __syncthreads();
   for (int t = threadIdx.x; t < 3 * n; t += blockDim.x) {
-    DobjDev& D = P->dobj[t / 3];
-    if (t % 3 < D.num_faces && ((mv.turn && D.attached) || t / 3 == mv.tr)) dobj_face(D, t % 3);
+    const DobjDev& D = src->dobj[t / 3];
+    if (t % 3 >= D.num_faces) continue;
+    if ((mv.turn && D.attached) || t / 3 == mv.tr) {
+      dobj_face(dst->dobj[t / 3], t % 3);
+    } else if (dst != src) {
+      Surface& F = dst->dobj[t / 3].faces[t % 3];
+      F.centroid = D.faces[t % 3].centroid;
+      F.normal = D.faces[t % 3].normal;
+      F.area = D.faces[t % 3].area;
+    }
   }
 }
 constexpr int kMoveThreads = 288;   // 9 x kMaxDobj
 __global__ void __launch_bounds__(kMoveThreads)
-k_move_dobj(SimParams* P, DobjMove mv) { move_dobjs(P, mv); }
+k_move_dobj(const SimParams* src, SimParams* dst, DobjMove mv) { move_dobjs(src, dst, mv); }
 
 // ---------------------------------------------------------------------- step
 #ifndef BLAZE_STEP_MIN_BLOCKS
@@ -510,8 +520,8 @@ constexpr int kMaskBatch = 7;
 // As kernels of their own the two reductions took 7.8 us and the turn of eight
 // lifters (a thread per object) 12.5 us beside a step of 23 us: ball mill,
 // 60,000 spheres, 64 steps 2.43 -> 2.12 ms.
-__device__ __forceinline__ void step_tail(const StepTail& tail, double e_pp, double e_lift,
-                                          double e_surf) {
+__device__ __forceinline__ void step_tail(const StepTail& tail, const SimParams* params,
+                                          double e_pp, double e_lift, double e_surf) {
   __shared__ double sh[3][kEnergyBlock];
   __shared__ int last;
   const int t = threadIdx.x;
@@ -554,7 +564,7 @@ __device__ __forceinline__ void step_tail(const StepTail& tail, double e_pp, dou
     for (int q = 0; q < 3; ++q) acc[q] += __ldcg(tail.part + 3 * b + q);
   reduce(acc[0], acc[1], acc[2]);
   if (t < 3) tail.tally[t] += sh[t][0];
-  if (tail.next) move_dobjs(tail.params, tail.move);
+  if (tail.next) move_dobjs(params, tail.next, tail.move);
 }
 
 // kPack: contacts shared by a warp (see the ensembles' step): the lanes list
@@ -576,7 +586,7 @@ constexpr unsigned kAll = 0xffffffffu;
 // last block to finish over the blocks in their order, so the sums do not
 // depend on timing.  The last block also makes the next step's moves of the
 // volume objects when the step after this one is launched with it (tail.next):
-// no other block reads them any more.
+// into the copy of the parameters that the next step reads.
 // kFast: the particle-particle law in contracted form (law_pp_fast) and the
 // contact normal from an approximate reciprocal; contact tests, walls, volume
 // objects and the integrator are unchanged.  Not with kEnergy.
@@ -889,7 +899,7 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
     }
   }
   } while (false);
-  if constexpr (kEnergy) step_tail(tail, e_pp, e_lift, e_surf);
+  if constexpr (kEnergy) step_tail(tail, Pg, e_pp, e_lift, e_surf);
 }
 
 // ------------------------------------------------------------ energy tallies
@@ -1193,8 +1203,9 @@ void launch_energy_reduce(const double* eb, int n_max, const StepCtl* ctl, doubl
   k_energy_final<<<1, kEnergyBlock, 0, st>>>(part, nb, tally);
 }
 
-void launch_move_dobj(SimParams* dp, const DobjMove& mv, int n_dobj, cudaStream_t st) {
-  if (n_dobj > 0) k_move_dobj<<<1, kMoveThreads, 0, st>>>(dp, mv);
+void launch_move_dobj(const SimParams* src, SimParams* dst, const DobjMove& mv, int n_dobj,
+                      cudaStream_t st) {
+  if (n_dobj > 0) k_move_dobj<<<1, kMoveThreads, 0, st>>>(src, dst, mv);
 }
 
 void launch_rotate_wobj(WallOp* ops, int n_ops, uint32_t rot_mask, float about_x, float about_y,

@@ -192,15 +192,14 @@ struct DobjMove {
 };
 // Work of the last block of a step that tallies energy (done: a zeroed
 // counter): tally[c] += the step's values, in a fixed order (part: 3 doubles
-// per block of kEnergyBlock particles), and with `next` the moves that the
-// following step starts with.
+// per block of kEnergyBlock particles), and with `next` (not the step's own
+// parameters) the moves that the following step starts with, written there.
 struct StepTail {
   unsigned int* done;
   double* part;
   double* tally;
-  SimParams* params;
+  SimParams* next;
   DobjMove move;
-  int next;
 };
 constexpr int kEnergyBlock = 256;
 // energy: the step tallies energy (with the reference's arithmetic).  fast:
@@ -210,15 +209,17 @@ void launch_step(const SimParams* dp, const WallOp* ops, WallGrid wg, const Stat
                  NbrList nl, StepCtl* ctl, StepLink link, bool spin_free,
                  const ForceCapture* cap, bool energy, const StepTail& tail, bool fast,
                  cudaStream_t st);
-// Polyhedra: tally[c] += sum of eb[c * n_max + i] over the current
-// particles, in the same order; part as in StepTail.
 // Self-check of div3_rn against IEEE division on n random triples:
 // *bad += the components that differ.
 void launch_check_div(long long n, unsigned long long seed, unsigned long long* bad,
                       cudaStream_t st);
+// Polyhedra: tally[c] += sum of eb[c * n_max + i] over the current
+// particles, in the same order; part as in StepTail.
 void launch_energy_reduce(const double* eb, int n_max, const StepCtl* ctl, double* part,
                           double* tally, cudaStream_t st);
-void launch_move_dobj(SimParams* dp, const DobjMove& mv, int n_dobj, cudaStream_t st);
+// (src and dst may be the same)
+void launch_move_dobj(const SimParams* src, SimParams* dst, const DobjMove& mv, int n_dobj,
+                      cudaStream_t st);
 // One step of the turn of the rotating world objects (bit k of rot_mask:
 // world object k) on the wall program.
 void launch_rotate_wobj(WallOp* ops, int n_ops, uint32_t rot_mask, float about_x, float about_y,
