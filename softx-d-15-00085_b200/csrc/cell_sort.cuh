@@ -8,8 +8,8 @@
 //   count   (in the caller's key kernel, cell_count): every particle's
 //           arrival number in its cell, the members per cell and per tile of
 //           kTileCells cells
-//   scan    (k_cell_scan) a block per tile: the members of the tiles before
-//           it, then the exclusive scan of its own cells -> start[]; the
+//   scan    (k_cell_scan) a block per tile (or some): the members of the tiles
+//           before it, then the exclusive scan of its own cells -> start[]; the
 //           counts are zeroed for the next sort as they are read
 //   place   (k_cell_place) member[start[cell] + arrival] = particle: the
 //           cells' members together, in arrival order
@@ -35,6 +35,7 @@ constexpr int kSortThreads = 256;          // threads per block of the count and
 constexpr int kScanThreads = 512;
 constexpr int kScanItems = 8;
 constexpr int kTileCells = kScanThreads * kScanItems;
+constexpr uint32_t kScanBlocks = 2048;
 
 struct CellSort {
   uint32_t* key;      // per particle: its cell; ncell: outside the grid, ncell + 1: parked

@@ -2,9 +2,8 @@
 a stable sort by the reference's hash (particles outside the grid, then parked
 ones, behind the others in their order) and the clamped 27 cells scanned in
 y, z, x order, at the sizes where the counting sort and the row search can go
-wrong: one block of particles and its edges, a tile of cells and its edges, radii
-that reach a few or all of their cells,
-grids whose hash aliases (x + z ncz + y ncx ncz with ncx != ncz), grids too
+wrong: one block of particles and its edges, a tile of cells and its edges, more
+tiles than the scan has blocks, radii that reach a few or all of their cells, whose hash aliases (x + z ncz + y ncx ncz with ncx != ncz), grids too
 small to leave cells out of the search, crowded cells."""
 import numpy as np
 import pytest
@@ -60,7 +59,8 @@ def definition(pos, pid, rad, origin, cell, nc, skin):
     (1, (3, 3, 3), 1.0, 0.0), (255, (7, 7, 7), 0.5, 0.0), (256, (16, 16, 16), 0.3, 0.0),
     (257, (15, 13, 21), 0.3, 0.0), (3000, (17, 15, 16), 0.9, 0.0), (3000, (16, 17, 16), 1.2, 0.05),
     (700, (12, 5, 2), 0.9, 0.0), (700, (2, 9, 11), 0.9, 0.0), (400, (1, 1, 1), 0.1, 0.0),
-    (2000, (64, 2, 64), 1.1, 0.0), (1500, (9, 9, 9), 1.3, 0.1), (5000, (40, 40, 40), 1.0, 0.0)])
+    (2000, (64, 2, 64), 1.1, 0.0), (1500, (9, 9, 9), 1.3, 0.1), (5000, (40, 40, 40), 1.0, 0.0),
+    (2000, (211, 204, 210), 1.0, 0.0), (3000, (211, 204, 210), 0.06, 0.0)])
 def test_order_and_list_by_definition(tmp_path, n, nc, fill, skin):
     rad = 0.1
     P, _ = synth.box_project(str(tmp_path), n_side=(2, 2, 2), radius=rad)
