@@ -3,7 +3,8 @@ a stable sort by the reference's hash (particles outside the grid, then parked
 ones, behind the others in their order) and the clamped 27 cells scanned in
 y, z, x order, at the sizes where the counting sort and the row search can go
 wrong: one block of particles and its edges, a tile of cells and its edges, more
-tiles than the scan has blocks, radii that reach a few or all of their cells, whose hash aliases (x + z ncz + y ncx ncz with ncx != ncz), grids too
+tiles than the scan has blocks, radii that reach a few or all of their cells,
+grids whose hash aliases (x + z ncz + y ncx ncz with ncx != ncz), grids too
 small to leave cells out of the search, crowded cells."""
 import numpy as np
 import pytest
