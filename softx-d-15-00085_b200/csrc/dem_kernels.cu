@@ -522,7 +522,7 @@ constexpr int kMaskBatch = 7;
 // 60,000 spheres, 64 steps 2.43 -> 2.12 ms.
 __device__ __forceinline__ void step_tail(const StepTail& tail, const SimParams* params,
                                           double e_pp, double e_lift, double e_surf) {
-  __shared__ double sh[3][kEnergyBlock];
+  __shared__ double sh[3][kEnergyBlock], sum[3];
   __shared__ int last;
   const int t = threadIdx.x;
   // the block's sums into tail.part, or the totals into tail.tally
@@ -531,27 +531,21 @@ __device__ __forceinline__ void step_tail(const StepTail& tail, const SimParams*
     sh[1][t] = b;
     sh[2][t] = c;
     __syncthreads();
-    for (int w = kEnergyBlock / 2; w >= 32; w >>= 1) {
-      if (t < w)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) sh[q][t] += sh[q][t + w];
-      __syncthreads();
-    }
-    if (t < 32) {
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        double v = sh[q][t];
-        for (int w = 16; w > 0; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w);
-        if (t == 0) sh[q][0] = v;
-      }
+    // a warp per sum; the pairs of a tree that halves the block each time
+    if (t < 96) {
+      const double* x = sh[t >> 5] + (t & 31);
+      double v = ((x[0] + x[128]) + (x[64] + x[192])) + ((x[32] + x[160]) + (x[96] + x[224]));
+      for (int w = 16; w > 0; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w);
+      if ((t & 31) == 0) sum[t >> 5] = v;
     }
     __syncthreads();
   };
+  static_assert(kEnergyBlock == 256, "the tree of a block's sums");
   reduce(e_pp, e_lift, e_surf);
-  if (t < 3) tail.part[3 * blockIdx.x + t] = sh[t][0];
-  __threadfence();
-  __syncthreads();
   if (t == 0) {
+    // (a fence of the whole block would wait for its state to be written)
+    for (int q = 0; q < 3; ++q) tail.part[3 * blockIdx.x + q] = sum[q];
+    __threadfence();
     last = atomicAdd(tail.done, 1u) == gridDim.x - 1u;
     if (last) *tail.done = 0u;
   }
@@ -563,7 +557,7 @@ __device__ __forceinline__ void step_tail(const StepTail& tail, const SimParams*
 #pragma unroll
     for (int q = 0; q < 3; ++q) acc[q] += __ldcg(tail.part + 3 * b + q);
   reduce(acc[0], acc[1], acc[2]);
-  if (t < 3) tail.tally[t] += sh[t][0];
+  if (t < 3) tail.tally[t] += sum[t];
   if (tail.next) move_dobjs(params, tail.next, tail.move);
 }
 
@@ -572,11 +566,12 @@ __device__ __forceinline__ void step_tail(const StepTail& tail, const SimParams*
 // belong to, and each particle adds up its own in slot order.  It pays where
 // the step is bound by one warp's chain of contacts: with the reference's
 // arithmetic below 57,000 particles (fewer per warp, warp_particles; one call
-// of one step of 10,000 19.7 -> 17.7 us) and with energy tallies (mill, 60,000, 64
-// steps 2.12 -> 2.05 ms).  On a full GPU a lane's own walk is as fast or faster:
-// 100,000 spheres, 16 steps, 0.304 against 0.300 ms; 1,000,000 in reference mode
-// 0.322 against 0.334, and with the contracted law, which is short, 16 steps 1.83
-// against 1.95 ms.
+// of one step of 10,000 19.7 -> 17.7 us) and with energy tallies up to 100,000
+// (mill, 60,000, 64 steps 2.12 -> 2.05 ms).  On a full GPU a lane's own walk is as
+// fast or faster: 100,000 spheres, 16 steps, 0.304 against 0.300 ms; 1,000,000 in
+// reference mode 0.322 against 0.334, with the contracted law, which is short, 16
+// steps 1.83 against 1.95 ms, and with tallies 229 against 245 us a step (in a
+// loose bed 60 against 68); 120,000 with tallies 41.5 against 42.8.
 constexpr int kPairChunk = 96;   // contacts in shared memory at a time
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -1168,7 +1163,8 @@ void launch_step(const SimParams* dp, const WallOp* ops, WallGrid wg, const Stat
   static_assert(kThreads == kEnergyBlock, "energy blocks");
   // (the energy sums are over kEnergyBlock consecutive particles)
   const int wp = energy ? 32 : warp_particles(n_max);
-  const bool pack = energy || (!fast && wp < 32);
+  // kPack: see k_step
+  const bool pack = energy ? n_max <= 100000 : !fast && wp < 32;
   const int g = pack ? warp_blocks(n_max, wp, kThreads) : blocks(n_max);
 #define BLAZE_STEP_ARGS dp, ops, wg, in_plain, in_sorted, out, ob, n_max, wp, nl, ctl, link, c, tail
 #define BLAZE_STEP(C, S, E, F, K) k_step<C, S, E, F, K><<<g, kThreads, 0, st>>>(BLAZE_STEP_ARGS)
@@ -1182,7 +1178,8 @@ void launch_step(const SimParams* dp, const WallOp* ops, WallGrid wg, const Stat
       else BLAZE_STEP(false, true, E, F, K);            \
     }                                                   \
   } while (0)
-  if (energy) BLAZE_STEP_CS(true, false, true);
+  if (energy && pack) BLAZE_STEP_CS(true, false, true);
+  else if (energy) BLAZE_STEP_CS(true, false, false);
   else if (fast) BLAZE_STEP_CS(false, true, false);
   else if (pack) BLAZE_STEP_CS(false, false, true);
   else BLAZE_STEP_CS(false, false, false);
