@@ -200,6 +200,12 @@ void build_params(blaze_sim* s) {
     T.d_kn = o.Dsurface_Kn; T.d_cn = o.Dsurface_Cn; T.d_muk = o.Dsurface_Fric_kinetic;
     for (int q = 0; q < kMaxPP; ++q) T.pp[q] = o.PP[q];
   }
+  // a contact's tangential factor depends on the two types only; its division
+  // here gives the device's bits (IEEE single precision, tangential_prefactor)
+  for (TypeParams& A : P.types)
+    for (int t = 0; t < kMaxTypes; ++t)
+      A.tan_pre[t] = (((0.50f * (A.mass + P.types[t].mass)) / P.dt) * 0.050f) *
+                     A.pp[t < kMaxPP ? t : 0].Fric_kinetic;
   P.n_dobj = s->n_d;
   for (int k = 0; k < s->n_d; ++k) {
     const DOBJ& D = s->d[k];

@@ -76,6 +76,7 @@ struct TypeParams {
   float s_kn, s_cn, s_mus, s_muk;
   float d_kn, d_cn, d_muk;
   PP_Parms pp[kMaxPP];
+  float tan_pre[kMaxTypes];   // tangential_prefactor against every type, by the host
 };
 
 struct DobjDev {
@@ -160,7 +161,7 @@ __device__ __forceinline__ float2 cell_gap(float p, float o, float cell, int g, 
 // a zero less one wrap to the largest word; those of a NaN are above the limit):
 // with a test and two selects for each component a step of 100,000 spheres in
 // the reference's arithmetic took 19.0 us instead of 16.3 (which has the
-// prefactors of k_step's sTan too).  Zeros are inside because a wall contact's
+// tangential factors by type too).  Zeros are inside because a wall contact's
 // tangential velocity has them (with them outside, one step of 10,000 17.8 us
 // instead of 17.4).
 // blaze_check_division compares it with IEEE division on the GPU.

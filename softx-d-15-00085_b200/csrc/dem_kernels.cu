@@ -591,6 +591,7 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
        StateBuf in_plain, StateBuf in_sorted, StateBuf out, OrderBuf ob, int n_max, int wp,
        NbrList nl, StepCtl* ctl, StepLink link, ForceCapture cap, StepTail tail) {
   __shared__ TypeParams sT[kMaxTypes];
+  const SimParams& P = *Pg;
   {
     const int words = (int)(sizeof(TypeParams) * kMaxTypes / 4);
     const int* src = reinterpret_cast<const int*>(Pg->types);
@@ -598,20 +599,6 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
     for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = src[k];
   }
   __syncthreads();
-  const SimParams& P = *Pg;
-  // The tangential factor of a contact (it has a division) depends on the two types
-  // only: a table per block where a lane walks its own contacts.  A step whose
-  // contacts are few and shared by a warp does not win back the table's wait
-  // (one step of 10,000: 18.0 us with it, 17.8 without).
-  constexpr bool kTan = !kFast && !kPack;
-  __shared__ float sTan[kTan ? kMaxTypes : 1][kMaxTypes];
-  if constexpr (kTan) {
-    for (int k = threadIdx.x; k < kMaxTypes * kMaxTypes; k += blockDim.x) {
-      const int a = k / kMaxTypes, b = k % kMaxTypes;
-      sTan[a][b] = tangential_prefactor(P, sT[a].pp[b < kMaxPP ? b : 0], sT[a].mass, sT[b].mass);
-    }
-    __syncthreads();
-  }
   const bool rebuilt = *link.rebuilt != 0;
   const StateBuf in = rebuilt ? in_sorted : in_plain;
   const int n = ctl->n_cur;
@@ -704,7 +691,7 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
       } else {
         const float3 nrm = div3_rn(rel, dist);   // = rel / dist, three correctly rounded quotients
         F = law_pp_pre<kSpin>(P, va - vb, nrm, dis, (-1.0f * nrm) * ra, nrm * pb4.w, wa, xyz(wb4),
-                              pp, va, vb, sTan[ta & (kMaxTypes - 1)][tb & (kMaxTypes - 1)],
+                              pp, va, vb, TA.tan_pre[tb & (kMaxTypes - 1)],
                               kEnergy ? &ec : nullptr);
       }
       f = f + F.trans;
@@ -759,9 +746,9 @@ k_step(const SimParams* __restrict__ Pg, const WallOp* __restrict__ ops, WallGri
         const TypeParams& TO = sT[__float_as_int(vo4.w) & (kMaxTypes - 1)];
         const float3 nrm = div3_rn(rel, dist);   // = rel / dist, three correctly rounded quotients
         float en = 0.0f;
-        const Forces F = law_pp<kSpin>(P, vo - vj, nrm, dis, (-1.0f * nrm) * xo.w, nrm * xj.w, xyz(wo4),
-                                       xyz(wj4), TO.pp[tb < kMaxPP ? tb : 0], vo, vj, TO.mass,
-                                       sT[tb & (kMaxTypes - 1)].mass, kEnergy ? &en : nullptr);
+        const Forces F = law_pp_pre<kSpin>(P, vo - vj, nrm, dis, (-1.0f * nrm) * xo.w, nrm * xj.w,
+                                           xyz(wo4), xyz(wj4), TO.pp[tb < kMaxPP ? tb : 0], vo, vj,
+                                           TO.tan_pre[tb & (kMaxTypes - 1)], kEnergy ? &en : nullptr);
         law[r] = F.trans.x;
         law[kPairChunk + r] = F.trans.y;
         law[2 * kPairChunk + r] = F.trans.z;
