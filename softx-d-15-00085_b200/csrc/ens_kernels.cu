@@ -725,47 +725,95 @@ __device__ __forceinline__ float ens_particle_step(const EnsGeom& g, const EnsBu
     int best = -1;
     float best_d = 0.0f;
     bool face = false;
+    // most of a cell's triangles are out of reach: a sphere around each (tri_bound)
+    // tells.  Its radius is rounded up by the coordinates' size, the sum by 1e-6:
+    // the FP32 distance and square are off by 2e-7 of the sum, which a large
+    // sphere at a small mesh near the origin would see.
+    auto touches_tri = [&](uint32_t q, float3 pp, float rp, float& delta, int& region) -> bool {
+      const float4 bs = __ldg(g.stri_b + q);
+      const float3 dc = pp - xyz(bs);
+      const float reach = (bs.w + rp) * (1.0f + 1e-6f);
+      float3 nrm;
+      return !(dot3(dc, dc) > reach * reach) &&
+             wall_touch<kCurved>(g.walls[__ldg(g.stri_ids + q)], pp, rp, nrm, delta, region);
+    };
+    // the warp's 32 tests at candidates q0 .. of particle src, whose list begins at c0
+    auto take = [&](int src, uint32_t q0, uint32_t c0, bool hit, int region, float delta) {
+      const unsigned on_face = __ballot_sync(kAll, hit && region == 0);
+      // overlaps are positive: their bits sort as they do; the first of equals
+      const uint32_t depth = hit && region != 0 ? __float_as_uint(delta) : 0u;
+      const uint32_t most = __reduce_max_sync(kAll, depth);
+      const int first = __ffs(__ballot_sync(kAll, depth == most)) - 1;
+      if (lane == src) {
+        if (on_face) face = true;
+        if (q0 == c0) keep = on_face;
+        if (most && (best < 0 || __uint_as_float(most) > best_d)) {
+          best = (int)(q0 - c0) + first;
+          best_d = __uint_as_float(most);
+        }
+      }
+    };
     // A particle's candidates are tested by the whole warp, one per lane: few of
     // a warp's particles are near the mesh, and with each tested by its own lane
     // the others wait for a chain of dependent loads: mixed charge of 21,000, 32
     // steps, 1.41 -> 1.25-1.30 ms (alone 3.04 -> 2.66); 100,000 spheres in a drum
-    // of 16,384 triangles 23.0 -> 19.3 us a step.
-    for (unsigned near = __ballot_sync(kAll, o1 > o0); near; near &= near - 1u) {
-      const int src = __ffs(near) - 1;
-      const uint32_t c0 = __shfl_sync(kAll, o0, src), c1 = __shfl_sync(kAll, o1, src);
-      const float rp = __shfl_sync(kAll, ra, src);
-      const float3 pp = f3(__shfl_sync(kAll, pd.x, src), __shfl_sync(kAll, pd.y, src),
-                           __shfl_sync(kAll, pd.z, src));
-      for (uint32_t q0 = c0; q0 < c1; q0 += 32u) {
-        const uint32_t q = q0 + (uint32_t)lane;
-        bool hit = false;
+    // of 16,384 triangles 23.0 -> 19.3 us a step.  Where a warp lies on the mesh and
+    // that takes more turns than the longest list, every lane tests its own: such
+    // warps are the last to end (hopper of 400,000, one alone, 148 -> 122 us a step,
+    // of 150,000 85 -> 77).  Not in a turning drum or among polyhedra, whose builds
+    // it only slows (drum 12.8 -> 13.5 us, mixed charge 67.7 -> 68.7).
+    unsigned near = __ballot_sync(kAll, o1 > o0);
+    if constexpr (kRot || kMix) {
+      for (; near; near &= near - 1u) {
+        const int src = __ffs(near) - 1;
+        const uint32_t c0 = __shfl_sync(kAll, o0, src), c1 = __shfl_sync(kAll, o1, src);
+        const float rp = __shfl_sync(kAll, ra, src);
+        const float3 pp = f3(__shfl_sync(kAll, pd.x, src), __shfl_sync(kAll, pd.y, src),
+                             __shfl_sync(kAll, pd.z, src));
+        for (uint32_t q0 = c0; q0 < c1; q0 += 32u) {
+          const uint32_t q = q0 + (uint32_t)lane;
+          int region = 0;
+          float delta = 0.0f;
+          const bool hit = q < c1 && touches_tri(q, pp, rp, delta, region);
+          take(src, q0, c0, hit, region, delta);
+        }
+      }
+    } else {
+      const bool own = __reduce_max_sync(kAll, o1 - o0) <=
+                       __reduce_add_sync(kAll, (o1 - o0 + 31u) / 32u);
+      int src = lane;
+      uint32_t q0 = o0, c0 = o0, c1 = own ? o1 : o0;
+      float rp = ra;
+      float3 pp = pd;
+      for (;;) {
+        if (own) {
+          if (!__any_sync(kAll, q0 < c1)) break;
+        } else if (q0 >= c1) {   // the same in every lane
+          if (!near) break;
+          src = __ffs(near) - 1;
+          near &= near - 1u;
+          q0 = c0 = __shfl_sync(kAll, o0, src);
+          c1 = __shfl_sync(kAll, o1, src);
+          rp = __shfl_sync(kAll, ra, src);
+          pp = f3(__shfl_sync(kAll, pd.x, src), __shfl_sync(kAll, pd.y, src),
+                  __shfl_sync(kAll, pd.z, src));
+        }
+        const uint32_t q = own ? q0 : q0 + (uint32_t)lane;
         int region = 0;
         float delta = 0.0f;
-        if (q < c1) {
-          // most of a cell's triangles are out of reach: a sphere around each
-          // (tri_bound) tells.  Its radius is rounded up by the coordinates'
-          // size, the sum by 1e-6: the FP32 distance and square are off by 2e-7
-          // of the sum, which a large sphere at a small mesh near the origin
-          // would see.
-          const float4 bs = __ldg(g.stri_b + q);
-          const float3 dc = pp - xyz(bs);
-          const float reach = (bs.w + rp) * (1.0f + 1e-6f);
-          float3 nrm;
-          if (!(dot3(dc, dc) > reach * reach))
-            hit = wall_touch<kCurved>(g.walls[__ldg(g.stri_ids + q)], pp, rp, nrm, delta, region);
-        }
-        const unsigned on_face = __ballot_sync(kAll, hit && region == 0);
-        // overlaps are positive: their bits sort as they do; the first of equals
-        const uint32_t depth = hit && region != 0 ? __float_as_uint(delta) : 0u;
-        const uint32_t most = __reduce_max_sync(kAll, depth);
-        const int first = __ffs(__ballot_sync(kAll, depth == most)) - 1;
-        if (lane == src) {
-          if (on_face) face = true;
-          if (q0 == c0) keep = on_face;
-          if (most && (best < 0 || __uint_as_float(most) > best_d)) {
-            best = (int)(q0 - c0) + first;
-            best_d = __uint_as_float(most);
+        const bool hit = q < c1 && touches_tri(q, pp, rp, delta, region);
+        if (own) {
+          if (hit && region == 0) {
+            face = true;
+            if (q - o0 < 32u) keep |= 1u << (q - o0);
+          } else if (hit && (best < 0 || delta > best_d)) {
+            best = (int)(q - o0);
+            best_d = delta;
           }
+          ++q0;
+        } else {
+          take(src, q0, c0, hit, region, delta);
+          q0 += 32u;
         }
       }
     }

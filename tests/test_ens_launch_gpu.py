@@ -156,3 +156,31 @@ def test_recorded_run(wp):
     adj.close()
     ens.close()
     o.close()
+
+
+@pytest.mark.parametrize("side", [0.09, 0.15, 0.3, 0.8])
+def test_warps_that_lie_on_a_mesh(side):
+    """A layer on a floor of triangles: lists of several windows, tested by the
+    warp or by each lane (shorter ones), also past their first 32 entries, and
+    contacts on faces, edges and vertices."""
+    r, n = 0.2, 64
+    g = np.arange(n)
+    rng = np.random.default_rng(7)
+    pos = np.stack([(g % 8) * 0.41 + 0.3, (g // 8) * 0.41 + 0.3, np.full(n, r - 2e-4)], 1)
+    pos[:, :2] += rng.uniform(-2e-3, 2e-3, (n, 2))
+    m = int(math.ceil(3.6 / side))
+    x = np.linspace(0.0, 3.6, m + 1)
+    z = 0.02 * ((np.add.outer(np.arange(m + 1), np.arange(m + 1)) % 3) == 0) if side > 0.2 else \
+        np.zeros((m + 1, m + 1))
+    W = [w for k, w in enumerate(synth.box_walls(3.6, 3.0)) if k != 4]
+    for i in range(m):
+        for j in range(m):
+            a, b = (x[i], x[j], z[i, j]), (x[i + 1], x[j], z[i + 1, j])
+            c, d = (x[i + 1], x[j + 1], z[i + 1, j + 1]), (x[i], x[j + 1], z[i, j + 1])
+            W += [E.triangle(a, b, c), E.triangle(a, c, d)]
+    S = synth.box_system(n, 3.6, 3.0, 0.45, 0, density=2500e-6, kn=1e5, restitution=0.6, mu=0.4)
+    S.nwalls, S.tri0, S.ntris = 5, 5, len(W) - 5
+    vel = rng.normal(scale=20.0, size=pos.shape).astype(np.float32)
+    for wp in (4, 32):
+        both([S], W, pos.astype(np.float32), np.full(n, r, np.float32), vel, E.LAW_LINEAR,
+             dict(warp_particles=wp), (1, 60), dt=5e-6, skin=0.02)

@@ -28,9 +28,9 @@ def lattice(n, pitch, origin, seed):
     return p[rng.permutation(n)].astype(np.float32), rng, m * pitch
 
 
-# the tallies' block sums: one size above a block, and many blocks
+# the tallies' block sums: one size above a block, many blocks, and without shared contacts
 @pytest.mark.parametrize("n,energy", [(n, False) for n in (1, 33, 257, 14208, 14209, 28417, 56832, 56833)] +
-                         [(n, True) for n in (257, 14209, 56833)])
+                         [(n, True) for n in (257, 14209, 56833, 100000, 100001)])
 def test_sphere_step_sizes(tmp_path, n, energy):
     r = 0.1
     P, _ = synth.box_project(str(tmp_path), n_side=(2, 2, 2), radius=r)
