@@ -24,7 +24,7 @@
 namespace blaze {
 
 // Warps that take a polyhedron (an SM holds 16 warps of 128 registers): four up
-// to two waves of blocks, two up to four waves, else one.  More warps shorten a rock's chain of tests
+// to two waves of blocks, two up to five waves, else one.  More warps shorten a rock's chain of tests
 // and take other rocks' places.  Time of k_mix_poly_step in us with 4, 2 and 1
 // warps a rock:
 //   drum, 1,000 rocks among 20,000 balls   40.1  39.9  48.4
@@ -33,9 +33,10 @@ namespace blaze {
 //   settled box of 8,000                   58.2  44.8  50.3   loose 56.4 42.3 29.1
 //   settled box of 16,000                 101.0  77.8  55.0   loose 95.1 73.2 44.2
 // and a whole step with 4 and 2, alone: 200 rocks among 4,000 balls 44.5 and
-// 50.1, 1,000 among 20,000 70.7 and 73.9.
+// 50.1, 1,000 among 20,000 70.7 and 73.9; with 2 and 1, 5,000 among 100,000 in the
+// drum 128 and 138.
 inline int mix_warps(int npoly) {
-  return npoly <= 2 * 148 * 4 ? 4 : (npoly <= 4 * 148 * 8 ? 2 : 1);
+  return npoly <= 2 * 148 * 4 ? 4 : (npoly <= 5 * 148 * 8 ? 2 : 1);
 }
 
 // Staged polyhedra -> the state right after blaze_ens_set_state (memory
