@@ -1,4 +1,4 @@
-"""The integration of INTEGRATION.md section 1, built: the reference's own
+"""The drop-in integration, built: the reference's own
 KDevice wrapper (Interface/KDevice.cpp, compiled unchanged against
 include/kdevice/Device/DeviceInterface.h) and project reader
 (Input/KSimulationData.cpp), linked with a headless driver against
