@@ -614,10 +614,11 @@ int build_if_graph(blaze_ens* e, int c) {
 //   box of  800,000   31.4 (35.1)  38.1 (33.0)
 //   box of 1,300,000  49.2 (54.7)  53.9 (49.8)
 // With triangles, cylinders or polyhedra a step is longer and re-sorts more often:
-//   hopper of  50,000  48.9 (28.2)  53.5 (27.3)
-//   hopper of 150,000  85.3 (50.5)  89.5 (49.8)
-//   hopper of 400,000 143.8 (82.1) 146.0 (79.2)
-//   drum mesh, 100,000 12.2         19.3
+//   hopper of  50,000  49.3 (28.8)  54.3 (27.6)
+//   hopper of 150,000  72.7 (49.0)  77.5 (48.0)
+//   hopper of 400,000 122.1 (81.3) 125.5 (78.3)
+//   drum mesh, 100,000 12.8         19.3
+//   20,000 balls, 1,000 rocks 68.2 (31.2) 70.7 (31.7)
 // and a box of 20,000 that re-sorts every 1, 2, 5 and 15 steps: 68.9, 35.9, 21.5
 // and 9.8 in rounds, 57.6, 35.0, 22.0 and 15.7 with IF nodes (92.8, 47.3, 21.4
 // and 9.8 without the short rounds).
